@@ -123,6 +123,7 @@ struct adg_ctx {
   adg_config cfg{};
   const KernelSet* ks = nullptr;
   int E = 0;  // elements per predictor block
+  bool E_default = true;  // neither the caller nor the autotuner chose E: it follows the layout's size
   int sweeps = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -304,6 +305,7 @@ int upload_tables(adg_ctx* ctx, const RemapTable* rm = nullptr) {
   const int D = ctx->cfg.D, Q = ks->Q;
   const size_t ne = H.n_elem();
   const size_t nf = H.face_left.size();
+  if (ctx->E_default) ctx->E = default_elems_per_block(*ks, (long long)ne);
   ADG_CUDA(ctx->Rvol.ensure(ne * Q * ks->Np_s), "alloc Rvol");
   ADG_CUDA(ctx->Tr.ensure(ne * 2 * D * (size_t)ks->TR_TILE), "alloc traces");
   ADG_CUDA(ctx->Fnum.ensure(nf * Q * (size_t)ks->NM), "alloc Fnum");
@@ -1201,10 +1203,8 @@ int adg_ctx_create(const adg_config* cfg, adg_ctx** out) {
   ctx->sweeps = cfg->picard_sweeps > 0 ? cfg->picard_sweeps : cfg->P;
   if (ctx->sweeps < 1) ctx->sweeps = 1;
   std::vector<int> ch = ks->elems_per_block_choices();
-  const int E0 = cfg->D == 2 ? 16 : 8;  // default where it is built, else the one choice of the configuration
-  ctx->E = (cfg->elems_per_block > 0 && std::find(ch.begin(), ch.end(), cfg->elems_per_block) != ch.end())
-               ? cfg->elems_per_block
-               : (std::find(ch.begin(), ch.end(), E0) != ch.end() ? E0 : ch.front());
+  ctx->E_default = !(cfg->elems_per_block > 0 && std::find(ch.begin(), ch.end(), cfg->elems_per_block) != ch.end());
+  ctx->E = ctx->E_default ? default_elems_per_block(*ks, 0) : cfg->elems_per_block;
   cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete ctx;
@@ -2249,7 +2249,10 @@ bool choice_built(const KernelSet* ks, int E) {
 static void apply_tuned_choices(adg_ctx* ctx) {
   if (ctx->cfg.elems_per_block > 0) return;
   int E = 0;
-  if (tune_lookup(tune_key(ctx, "plain"), &E) && choice_built(ctx->ks, E)) ctx->E = E;
+  if (tune_lookup(tune_key(ctx, "plain"), &E) && choice_built(ctx->ks, E)) {
+    ctx->E = E;
+    ctx->E_default = false;
+  }
   if (ctx->seed_mode && tune_lookup(tune_key(ctx, ctx->seed_mode == 2 ? "seeded_fp32" : "seeded_fp64"), &E) &&
       choice_built(ctx->ks, E))
     ctx->Es = E;
@@ -2304,10 +2307,12 @@ int adg_autotune(adg_ctx* ctx, int nsteps, int* E_out, double* ms, int cap) {
   size_t best = 0;
   for (size_t i = 1; i < ch.size(); ++i)
     if (t[i] < t[best]) best = i;
-  if (seeded)
+  if (seeded) {
     ctx->Es = ch[best];
-  else
+  } else {
     ctx->E = ch[best];
+    ctx->E_default = false;
+  }
   tune_store(tune_key(ctx, seeded ? (ctx->seed_mode == 2 ? "seeded_fp32" : "seeded_fp64") : "plain"), ch[best]);
   ctx->graph_stale = true;  // the captured step used the old choice
   if (E_out) *E_out = ch[best];

@@ -46,8 +46,57 @@ constexpr uint32_t kStatusNaN = 1u;
 constexpr uint32_t kStatusNonPositiveDensity = 2u;
 constexpr uint32_t kStatusPressureFloor = 4u;
 
-// Floor that keeps NaN (std::max(_prs, limit) semantics, Compressible_Euler.h:586).
-__device__ __forceinline__ double floor_limit(double p) { return (p < kPdeLimit) ? kPdeLimit : p; }
+// Reciprocal and square root with fewer FP64 operations: the FP32 estimate of
+// the significand (its bits moved by integer code; a conversion instruction
+// would occupy the FP64 pipe), then one third-order Householder step.  With
+// e = 1 - x r the estimate's relative error (about 2^-22),
+//   1/x = r (1 + e + e^2 + ..), sqrt(x) = x r (1 + e/2 + 3 e^2/8 + ..),
+// whose next terms are below 2^-65: the results are within one unit in the
+// last place.  3 and 5 FP64 operations; outside 2^-900 .. 2^900 (zero,
+// infinities, NaN, negative square roots) the operators.
+__device__ __forceinline__ float significand_f32(int hi, int lo, int exp_bits) {
+  return __int_as_float(exp_bits | ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29));
+}
+__device__ __forceinline__ double widen_f32(float r, int exp_add, int sign) {
+  const int b = __float_as_int(r);
+  return __hiloint2double(((b >> 3) + (exp_add << 20)) | sign, b << 29);
+}
+__device__ __forceinline__ double fast_rcp(double x) {
+  const int hi = __double2hiint(x), ef = (hi >> 20) & 0x7ff;
+  if ((unsigned)(ef - 123) > 1800u) return 1.0 / x;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(significand_f32(hi, __double2loint(x), 0x3f800000)));
+  const double r0 = widen_f32(r, 1023 - 127 + 1023 - ef, hi & (int)0x80000000);
+  const double e = fma(-x, r0, 1.0);
+  return fma(r0, fma(e, e, e), r0);
+}
+__device__ __forceinline__ double fast_sqrt(double x) {
+  const int hi = __double2hiint(x), ef = hi >> 20;  // negative numbers: ef < 0
+  if ((unsigned)(ef - 123) > 1800u) return sqrt(x);
+  const int k = ef - 1023, odd = k & 1;  // significand in [1, 4), even exponent
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(significand_f32(hi, __double2loint(x), 0x3f800000 + (odd << 23))));
+  const double r0 = widen_f32(r, 1023 - 127 - ((k - odd) >> 1), 0);
+  const double h = x * r0, e = fma(-h, r0, 1.0);
+  return fma(h, e * fma(0.375, e, 0.5), h);
+}
+__device__ __forceinline__ double reciprocal(double x) { return fast_rcp(x); }
+__device__ __forceinline__ float reciprocal(float x) { return 1.0f / x; }
+
+// Floor that keeps NaN (std::max(_prs, limit) semantics, Compressible_Euler.h:586);
+// in FP64 the comparison runs only near the floor (a comparison of the high
+// words decides above it).
+__device__ __forceinline__ double floor_limit(double p) {
+  constexpr int kAbove = 0x3ce50000;  // 2.33e-15, above the floor
+  if (__double2hiint(p) < kAbove) p = (p < kPdeLimit) ? kPdeLimit : p;
+  return p;
+}
+__device__ __forceinline__ float floor_limit(float p) { return (p < (float)kPdeLimit) ? (float)kPdeLimit : p; }
+// 1 / max(rho, floor) from the reciprocal at hand
+__device__ __forceinline__ double floored_reciprocal(double rho, double r) {
+  if (__double2hiint(rho) < 0x3ce50000) r = (rho < kPdeLimit) ? 1.0 / kPdeLimit : r;
+  return r;
+}
 
 // Physical flux of the compressible Euler equations in every direction at one
 // point (Compressible_Euler.h:370-487; pressure Compressible_Euler.h:562-589).
@@ -55,15 +104,14 @@ __device__ __forceinline__ double floor_limit(double p) { return (p < kPdeLimit)
 template <int D, class T = double>
 __device__ __forceinline__ void euler_flux_all(const T* u, T gm1, T* F) {
   constexpr int Q = D + 2;
-  const T r = T(1) / u[0];
+  const T r = reciprocal(u[0]);
   T v[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) v[d] = u[d + 1] * r;
   T ke = u[1] * v[0];
 #pragma unroll
   for (int d = 1; d < D; ++d) ke = fma(u[d + 1], v[d], ke);
-  T p = gm1 * fma(T(-0.5), ke, u[D + 1]);
-  p = (p < T(kPdeLimit)) ? T(kPdeLimit) : p;
+  const T p = floor_limit(gm1 * fma(T(-0.5), ke, u[D + 1]));
   const T ep = u[D + 1] + p;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
@@ -85,7 +133,7 @@ __device__ __forceinline__ void euler_flux_all(const T* u, T gm1, T* F) {
 // max(|un-c|, |un|, |un+c|) = |un| + c (Compressible_Euler.h:489-518, 591-604).
 template <int D>
 __device__ __forceinline__ double euler_flux_normal(int d, const double* u, double gamma, double* F) {
-  const double r = 1.0 / u[0];
+  const double r = fast_rcp(u[0]);
   double v[D];
 #pragma unroll
   for (int k = 0; k < D; ++k) v[k] = u[k + 1] * r;
@@ -93,8 +141,7 @@ __device__ __forceinline__ double euler_flux_normal(int d, const double* u, doub
 #pragma unroll
   for (int k = 1; k < D; ++k) ke = fma(u[k + 1], v[k], ke);
   const double p = floor_limit((gamma - 1.0) * fma(-0.5, ke, u[D + 1]));
-  // 1 / max(rho, floor) from the reciprocal already at hand
-  const double rinv_c = (u[0] < kPdeLimit) ? 1.0 / kPdeLimit : r;
+  const double rinv_c = floored_reciprocal(u[0], r);
   double vd = v[0], md = u[1];
 #pragma unroll
   for (int k = 1; k < D; ++k)
@@ -106,7 +153,7 @@ __device__ __forceinline__ double euler_flux_normal(int d, const double* u, doub
 #pragma unroll
   for (int k = 0; k < D; ++k) F[k + 1] = (k == d) ? fma(md, v[k], p) : md * v[k];
   F[D + 1] = (u[D + 1] + p) * vd;
-  const double c = sqrt(gamma * (p * rinv_c));
+  const double c = fast_sqrt(gamma * (p * rinv_c));
   return fabs(vd) + c;
 }
 
@@ -203,13 +250,13 @@ __device__ __forceinline__ float euler_dflux_normal(int d, const float* u, const
 // CFL speed max_d(|u_d/rho| + c) at one point (Compressible_Euler.cpp:57-70).
 template <int D>
 __device__ __forceinline__ double euler_cfl_lambda(const double* u, double gamma) {
-  const double r = 1.0 / u[0];
+  const double r = fast_rcp(u[0]);
   double ke = 0.0;
 #pragma unroll
   for (int d = 0; d < D; ++d) ke += (u[d + 1] * u[d + 1]) * r;
   const double p = floor_limit((gamma - 1.0) * (u[D + 1] - 0.5 * ke));
-  const double rinv_c = (u[0] < kPdeLimit) ? 1.0 / kPdeLimit : r;
-  const double c = sqrt(gamma * (p * rinv_c));
+  const double rinv_c = floored_reciprocal(u[0], r);
+  const double c = fast_sqrt(gamma * (p * rinv_c));
   double lam = fabs(u[1] * r) + c;
 #pragma unroll
   for (int d = 1; d < D; ++d) lam = fmax(lam, fabs(u[d + 1] * r) + c);

@@ -1,0 +1,158 @@
+// Fixed-point columns: the linear operators of the FP64 path on the integer
+// pipes.  GB300 issues 1.6 FP64 operations per clock and SM; beside them,
+// without slowing them, it issues about 42 32 x 32 + 64 -> 64 multiply-adds
+// and 64 to 128 shifts, adds and logic operations (measured).  The operators
+// of an element are linear maps with constant coefficients, so they run on
+// 64-bit integers with one exponent per (element, variable) column and leave
+// the FP64 pipe to the flux evaluations.
+//
+// A column value is v 2^(E - 1082) with |v| <= 2^60; the bound of the column
+// is 2^(E - 1022), so E compares with the exponent field of a double.  A
+// coefficient is a 60-bit fraction C = ch 2^30 + cl (cl signed), an operand is
+// split into v = h 2^30 + l, and c v = h ch + (h cl + l ch) / 2^30 takes three
+// multiply-adds: the dropped product l cl is below one unit of the result, so
+// a term's error is 2^-60 of the bound where the FP64 form's is 2^-53 of the
+// partial sum.  Conversions are integer code too (a hardware conversion
+// occupies the FP64 pipe).  NaN and infinities make a column's results NaN
+// (fx_poison); columns beyond 2^1017 likewise, columns of subnormal numbers
+// are zero.
+#pragma once
+
+#include <cstdint>
+
+namespace adg {
+
+constexpr int kFxLimb = 30;
+constexpr int kFxLow = (1 << kFxLimb) - 1;
+constexpr long long kFxHalf = 1LL << (kFxLimb - 1);  // half a unit of the sum of the middle products
+
+__device__ __forceinline__ int fx_hi(long long v) { return (int)(v >> kFxLimb); }
+__device__ __forceinline__ int fx_lo(long long v) { return (int)v & kFxLow; }
+
+// Limbs of a coefficient's 60-bit fraction.
+struct FxCoef {
+  int h, l;
+};
+
+// Sum of products.  A product adds at most 1.5 2^60 to the middle sum B: it
+// is folded after four.
+struct FxSum {
+  long long A = 0, B = kFxHalf;
+  __device__ __forceinline__ void add(long long v) { A += v; }
+  __device__ __forceinline__ void mul(int h, int l, int ch, int cl) {
+    A = (long long)h * ch + A;
+    B = (long long)h * cl + B;
+    B = (long long)l * ch + B;
+  }
+  __device__ __forceinline__ void mul(long long v, const FxCoef& c) { mul(fx_hi(v), fx_lo(v), c.h, c.l); }
+  // a compile-time coefficient: the dropped l cl made up for in the mean (l
+  // is uniform), which costs one constant per sum
+  __device__ __forceinline__ void mulc(int h, int l, int ch, int cl) {
+    mul(h, l, ch, cl);
+    B += cl >> 1;
+  }
+  __device__ __forceinline__ void fold() {
+    A += B >> kFxLimb;
+    B = 0;
+  }
+  __device__ __forceinline__ long long get() const { return A + (B >> kFxLimb); }
+};
+
+__device__ __forceinline__ int fx_exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// Quiet-NaN bits for every output of a column whose exponent is that of
+// infinities and NaN or leaves the range of doubles.
+constexpr int kFxMaxExp = 2039;
+constexpr int kFxNanExp = 4096;
+__device__ __forceinline__ int fx_poison(int E) { return E > kFxMaxExp ? 0x7ff80000 : 0; }
+
+// x as a column value of exponent E >= the exponent field of x (exact down to
+// 2^-7 of the bound, truncated toward zero below; a negative x one unit
+// lower: its complement, not its negative).
+__device__ __forceinline__ long long fx_from_double(double x, int E) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+  const unsigned long long m = ((unsigned long long)mh << 39) | ((unsigned long long)(unsigned)lo << 7);
+  const int r = E - ((hi >> 20) & 0x7ff);
+  const long long s = hi >> 31;  // 0 or -1
+  return (long long)(m >> (r < 63 ? r : 63)) ^ s;
+}
+
+// Column value to the nearest double (a negative one from its complement);
+// nan_bits: fx_poison of the column.  The common case has a bit set in the
+// high word and a column exponent whose doubles are normal.
+static __device__ __noinline__ double fx_to_double_small(long long v, int E, int nan_bits);
+__device__ __forceinline__ double fx_to_double(long long v, int E, int nan_bits) {
+  const int s = (int)(v >> 32) >> 31;
+  const unsigned hi = (unsigned)((int)(v >> 32) ^ s), lo = (unsigned)((int)v ^ s);
+  if (hi == 0 || E < 64) return fx_to_double_small(v, E, nan_bits);
+  const int n = __clz((int)hi);
+  const unsigned mh = __funnelshift_l(lo, hi, n), ml = lo << n;  // leading bit at 31
+  // significand with its leading bit, rounded; the bit adds one to the field
+  const unsigned long long d = ((((unsigned long long)mh << 32) | ml) >> 11) + ((ml >> 10) & 1u);
+  const int field = (E + 3 - n) << 20;
+  return __hiloint2double(((int)(d >> 32) + field) | (s & (int)0x80000000) | nan_bits, (int)d);
+}
+static __device__ __noinline__ double fx_to_double_small(long long v, int E, int nan_bits) {
+  const long long s = v >> 63;
+  const unsigned long long a = (unsigned long long)(v ^ s);
+  const int n = __clzll((long long)a);
+  const unsigned long long m = n < 64 ? a << n : 0;
+  const int ef = E + 3 - n;
+  unsigned long long d = (m >> 11) + ((m >> 10) & 1) + ((unsigned long long)(unsigned)ef << 52);
+  if (ef < 0 || (long long)m >= 0) d = 0;
+  return __hiloint2double((int)(d >> 32) | ((int)s & (int)0x80000000) | nan_bits, (int)d);
+}
+
+// v / 2, rounded.
+__device__ __forceinline__ long long fx_half(long long v) { return (v + 1) >> 1; }
+
+// v 2^-shift, truncated downward.
+__device__ __forceinline__ long long fx_align(long long v, int shift) { return v >> (shift < 63 ? shift : 63); }
+// the same for a shift of either sign
+__device__ __forceinline__ long long fx_move(long long v, int shift) {
+  return fx_align(v << (shift < 0 ? -shift : 0), shift > 0 ? shift : 0);
+}
+
+// A positive double as a 60-bit fraction times 2^(ef - 1022).
+struct FxFactor {
+  FxCoef c;
+  int ef;
+};
+__device__ __forceinline__ FxFactor fx_factor(double c) {
+  const int hi = __double2hiint(c), lo = __double2loint(c);
+  const unsigned long long m = ((unsigned long long)(((unsigned)hi & 0xfffffu) | 0x100000u) << 39) |
+                               ((unsigned long long)(unsigned)lo << 7);
+  return {{(int)(m >> kFxLimb), (int)m & kFxLow}, (hi >> 20) & 0x7ff};
+}
+__device__ __forceinline__ long long fx_scale(long long v, const FxFactor& f) {
+  FxSum s;
+  s.mul(v, f.c);
+  return s.get();
+}
+// Exponent of fx_scale's result for operands of exponent e + growth (beyond
+// every double's when the operands or the factor are not finite).
+__device__ __forceinline__ int fx_scaled_exp(int e, int growth, const FxFactor& f) {
+  return e > kFxMaxExp || f.ef == 2047 ? kFxNanExp : e + growth + f.ef - 1022;
+}
+
+// Exponent E with sum |x_n| <= 2^(E - 1022), x_n at stride s: the largest
+// exponent field plus what the sum of the truncated significands (20 bits,
+// rounded up) needs.  2047 (infinity or NaN) stays above kFxMaxExp.
+template <int N>
+__device__ __forceinline__ int fx_norm_exp(const double* x, int s) {
+  int top = 0;
+#pragma unroll 4
+  for (int n = 0; n < N; ++n) top = max(top, fx_exp_field(x[n * s]));
+  int sum = 0;
+#pragma unroll 4
+  for (int n = 0; n < N; ++n) {
+    const int hi = __double2hiint(x[n * s]);
+    const int r = top - ((hi >> 20) & 0x7ff);
+    sum += (int)((((unsigned)hi & 0xfffffu) | 0x100000u) >> (r < 31 ? r : 31)) + 1;
+  }
+  const int bits = 32 - __clz(sum);  // sum < 2^bits, in units of 2^(top - 1023 - 20)
+  return top + (bits > 21 ? bits - 21 : 0);
+}
+
+}  // namespace adg

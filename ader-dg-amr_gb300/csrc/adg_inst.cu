@@ -3,6 +3,7 @@
 // -DADG_NS (its namespace) and -DADG_FACTORY (factory function name).
 #include <atomic>
 #include "adg_kernelset.hpp"
+#include "adg_predictor_fx.cuh"
 #include ADG_HDR
 
 namespace adg {
@@ -11,7 +12,7 @@ namespace {
 using O = ADG_NS::Ops;
 
 // Dynamic shared memory of k_predictor per phase (ld = E Q + 1 slots per point):
-//   FP64 sweeps             D NQ_ST ld doubles   (MODE 0 first sweep: D NQ_INIT)
+//   FP64 sweeps             D NQ_ST ld doubles
 //   FP32 sweeps (MODE 2)    D NQ_S ld floats     (one time slice at a time)
 //   final volume slices     (1 + D) NQ_S ld doubles
 //   face traces             2 NQ_BD ld doubles   (one direction at a time)
@@ -47,38 +48,55 @@ cudaError_t ensure_smem_attr(std::atomic<unsigned long long>& mask, F* func, siz
   return e;
 }
 
+// Grid of a fallback pass over a list of at most n elements counted on the
+// device: two blocks per SM stride over it.
+int list_grid(int n, int E) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    sms = 152;
+  const int grid = (n + E - 1) / E;
+  return grid < 2 * sms ? grid : 2 * sms;
+}
+
+// Mode 0: the plain Picard path.
+template <int E>
+cudaError_t launch_plain(const PredictorArgs& a, cudaStream_t s) {
+  constexpr size_t smem = FxShape<O, E>::BYTES;
+  if (a.n_elem <= 0) return cudaSuccess;
+  if (a.elem_list && a.list_count) {
+    static std::atomic<unsigned long long> attr{0};
+    cudaError_t e = ensure_smem_attr(attr, k_predictor_fx_list<O, E>, smem);
+    if (e != cudaSuccess) return e;
+    k_predictor_fx_list<O, E><<<list_grid(a.n_elem, E), FxShape<O, E>::NT, smem, s>>>(a);
+  } else {
+    static std::atomic<unsigned long long> attr{0};
+    cudaError_t e = ensure_smem_attr(attr, k_predictor_fx<O, E>, smem);
+    if (e != cudaSuccess) return e;
+    k_predictor_fx<O, E><<<(a.n_elem + E - 1) / E, FxShape<O, E>::NT, smem, s>>>(a);
+  }
+  return cudaGetLastError();
+}
+
+// Modes 1 and 2 over the element range, mode 3 over a list counted on the
+// device.
 template <int E, int MODE>
 cudaError_t launch_predictor_mode(const PredictorArgs& a, cudaStream_t s) {
   constexpr size_t smem = smem_bytes<E, MODE>();
-  if (a.elem_list && a.list_count) {  // fallback pass (modes 0 and 3): two blocks per SM stride over the list
-    if constexpr (MODE == 0 || MODE == 3) {
-      static std::atomic<unsigned long long> attr{0};
-      cudaError_t e = ensure_smem_attr(attr, k_predictor_list<O, E, MODE>, smem);
-      if (e != cudaSuccess) return e;
-      int dev = 0, sms = 0;
-      if (cudaGetDevice(&dev) != cudaSuccess ||
-          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-        sms = 152;
-      int grid = (a.n_elem + E - 1) / E;
-      if (grid > 2 * sms) grid = 2 * sms;
-      if (grid <= 0) return cudaSuccess;
-      k_predictor_list<O, E, MODE><<<grid, E * O::Q, smem, s>>>(a);
-      return cudaGetLastError();
-    } else {
-      return cudaErrorInvalidValue;
-    }
-  }
+  static std::atomic<unsigned long long> attr{0};
+  if (a.n_elem <= 0) return cudaSuccess;
   if constexpr (MODE == 3) {
-    return cudaErrorInvalidValue;  // mode 3 runs on element lists only
+    if (!a.elem_list || !a.list_count) return cudaErrorInvalidValue;
+    cudaError_t e = ensure_smem_attr(attr, k_predictor_list<O, E, MODE>, smem);
+    if (e != cudaSuccess) return e;
+    k_predictor_list<O, E, MODE><<<list_grid(a.n_elem, E), E * O::Q, smem, s>>>(a);
   } else {
-    static std::atomic<unsigned long long> attr{0};
+    if (a.elem_list && a.list_count) return cudaErrorInvalidValue;
     cudaError_t e = ensure_smem_attr(attr, k_predictor<O, E, MODE>, smem);
     if (e != cudaSuccess) return e;
-    const int grid = (a.n_elem + E - 1) / E;
-    if (grid <= 0) return cudaSuccess;
-    k_predictor<O, E, MODE><<<grid, E * O::Q, smem, s>>>(a);
-    return cudaGetLastError();
+    k_predictor<O, E, MODE><<<(a.n_elem + E - 1) / E, E * O::Q, smem, s>>>(a);
   }
+  return cudaGetLastError();
 }
 
 // The learned-seed path (predictor modes 1-3, the fused TF32 inference) is
@@ -97,14 +115,14 @@ cudaError_t launch_predictor(const PredictorArgs& a, cudaStream_t s, int mode) {
   } else {
     if (mode != 0) return cudaErrorNotSupported;
   }
-  return launch_predictor_mode<E, 0>(a, s);
+  return launch_plain<E>(a, s);
 }
 
-// Elements per block of the plain-only configurations: the largest of 16, 8,
-// 4 whose FP64 sweep buffers fit the 227 KB of shared memory of a block.
-constexpr int lite_elems() {
-  return smem_bytes<16, 0>() <= 227 * 1024 ? 16 : smem_bytes<8, 0>() <= 227 * 1024 ? 8 : 4;
-}
+// Elements per block of the plain-only configurations: whole warps of columns
+// at D = 2 (a block of 16 at P = 6 needs 214 KB of shared memory), at D = 3
+// what leaves two blocks on an SM (P = 3, 20 x 14 x 18: 4 / 6 elements 692 /
+// 737 us).
+constexpr int lite_elems() { return O::D == 2 ? 8 : 4; }
 
 struct Impl final : KernelSet {
   Impl() {
@@ -123,14 +141,14 @@ struct Impl final : KernelSet {
   bool seed_modes() const override { return kSeedModes; }
 #if ADG_LITE
   std::vector<int> elems_per_block_choices() const override { return {lite_elems()}; }
-  size_t predictor_smem(int) const override { return smem_bytes<lite_elems(), 0>(); }
+  size_t predictor_smem(int) const override { return FxShape<O, lite_elems()>::BYTES; }
   cudaError_t predictor(const PredictorArgs& a, int, cudaStream_t s, int mode) const override {
     return launch_predictor<lite_elems()>(a, s, mode);
   }
 #elif ADG_D == 2
   std::vector<int> elems_per_block_choices() const override { return {8, 16, 32}; }
   size_t predictor_smem(int E) const override {
-    return E == 8 ? smem_bytes<8, 0>() : E == 16 ? smem_bytes<16, 0>() : smem_bytes<32, 0>();
+    return E == 8 ? FxShape<O, 8>::BYTES : E == 16 ? FxShape<O, 16>::BYTES : FxShape<O, 32>::BYTES;
   }
   cudaError_t predictor(const PredictorArgs& a, int E, cudaStream_t s, int mode) const override {
     if (E == 8) return launch_predictor<8>(a, s, mode);
@@ -138,11 +156,14 @@ struct Impl final : KernelSet {
     return launch_predictor<32>(a, s, mode);
   }
 #else
+  // (the plain path takes 6 elements for the choice 8: 30 columns fill a warp
+  // and its table reads are uniform; P = 2, 64^3: 9.0 -> 8.5 ms)
   std::vector<int> elems_per_block_choices() const override { return {4, 8, 16}; }
   size_t predictor_smem(int E) const override {
-    return E == 4 ? smem_bytes<4, 0>() : E == 8 ? smem_bytes<8, 0>() : smem_bytes<16, 0>();
+    return E == 4 ? FxShape<O, 4>::BYTES : E == 8 ? FxShape<O, 6>::BYTES : FxShape<O, 16>::BYTES;
   }
   cudaError_t predictor(const PredictorArgs& a, int E, cudaStream_t s, int mode) const override {
+    if (mode == 0 && E == 8) return launch_plain<6>(a, s);
     if (E == 4) return launch_predictor<4>(a, s, mode);
     if (E == 8) return launch_predictor<8>(a, s, mode);
     return launch_predictor<16>(a, s, mode);

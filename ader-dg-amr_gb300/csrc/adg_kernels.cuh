@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "adg_device.cuh"
+#include "adg_fx.cuh"
 
 namespace adg {
 
@@ -550,11 +551,11 @@ __device__ __forceinline__ void fp64_epilogue(const double* hw, const double* u,
   if constexpr (D == 3) face_traces<O, E, 2>(hw, sm, col, LD, a, e0, limit);
 }
 
-// MODE 0: plain FP64 Picard (the reference's initial guess, P sweeps);
 // MODE 1 / 2: seeded, `sweeps` sweeps from the learned seed in FP64 / FP32,
 // the first one judging the seed by its residual;
-// MODE 3: the FP64 Picard of MODE 0 with the final stage and split trace
-// tiles of MODE 2 (the fallback elements of a MODE 2 step).
+// MODE 3: the full Picard in FP64 with the final stage and split trace tiles
+// of MODE 2 (the fallback elements of a MODE 2 step).
+// (Mode 0, the plain path, is k_predictor_fx of adg_predictor_fx.cuh.)
 // Resident blocks per SM that MODE 2 asks for: 16 warps (at most 128
 // registers a thread); its sliced sweeps leave the shared memory for them.
 template <int E, int Q, int MODE>
@@ -598,7 +599,7 @@ __device__ __forceinline__ void predictor_chunk(const PredictorArgs& a, double* 
   float dlt[NP_ST];  // MODES 2, 3: H_w - W U in FP32
   float uf[NP_S];    // MODES 2, 3: U_w in FP32
 
-  if constexpr (MODE == 0 || MODE == 3) {
+  if constexpr (MODE == 3) {
     // ---- sweep 1: the reference's initial guess H_w = [U_w, 0, ...]
     // (AmrDG.tpp:520-533) does not depend on x_0; evaluate on the (x_1.., t) grid.
     O::vol_eval_init(RegIn{u}, ColOut{sm + col, LD});
@@ -736,11 +737,11 @@ __device__ __forceinline__ void predictor_chunk(const PredictorArgs& a, double* 
 }
 
 // The kernels: one element group per block over the element range
-// (k_predictor), or a short grid striding over the groups of an element
-// list whose length is known only on the device (k_predictor_list, the
-// fallback pass).  Every phase of a group ends with a barrier, so the next
+// (k_predictor, modes 1 and 2), or a short grid striding over the groups of an
+// element list whose length is known only on the device (k_predictor_list,
+// the fallback pass, mode 3).  Every phase of a group ends with a barrier, so the next
 // group may reuse the shared memory.
-template <class O, int E, int MODE = 0>
+template <class O, int E, int MODE>
 __global__ void __launch_bounds__(E * O::Q, (predictor_min_blocks<E, O::Q, MODE>()))
     k_predictor(PredictorArgs a) {
   extern __shared__ double sm[];

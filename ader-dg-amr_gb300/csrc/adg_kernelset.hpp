@@ -21,8 +21,9 @@ struct KernelSet {
   // the learned-seed predictor modes (1-3) are built for this (D, P)
   virtual bool seed_modes() const = 0;
   virtual size_t predictor_smem(int E) const = 0;
-  // mode 0: FP64 Picard; 1 / 2: seeded, FP64 / FP32 sweeps; 3: FP64 Picard with
-  // mode 2's final stage (element lists only: the fallback of a mode-2 step).
+  // mode 0: the plain Picard path; 1 / 2: seeded, FP64 / FP32 sweeps; 3: FP64
+  // Picard with mode 2's final stage (element lists only: the fallback of a
+  // mode-2 step).
   // An element list counted on the device (a.list_count, modes 0 and 3: the
   // fallback) is strided over by a short grid; one counted on the host
   // (a.list_count == nullptr, a.n_elem entries) runs one group per block.
@@ -58,6 +59,17 @@ const KernelSet* kernels_D2P4();
 const KernelSet* kernels_D2P5();
 const KernelSet* kernels_D2P6();
 const KernelSet* kernels_D3P3();
+
+// Elements per block where nothing else chose them.  D = 2: blocks of 8 while
+// blocks of 16 leave the SMs with a few blocks each (D2P3 step, us, 8 / 16:
+// 24^2 86 / 101, 48^2 96 / 102; 128^2 329 / 332; 256^2 1220 / 1169).
+inline int default_elems_per_block(const KernelSet& ks, long long n_elem) {
+  const std::vector<int> ch = ks.elems_per_block_choices();
+  const int E = ks.D == 2 && n_elem > 12288 ? 16 : 8;
+  for (int c : ch)
+    if (c == E) return E;
+  return ch.front();
+}
 
 inline const KernelSet* kernel_set(int D, int P) {
   if (D == 2 && P == 1) return kernels_D2P1();

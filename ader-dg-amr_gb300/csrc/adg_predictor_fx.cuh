@@ -1,0 +1,803 @@
+// Plain Picard predictor (AmrDG.tpp:495-537, 744-827) with its linear
+// operators in fixed point (adg_fx.cuh) and its fluxes in FP64.
+//
+// A block holds E elements, C = E Q columns, and gives every column
+// N^(D-1) threads, one per line of points along x_0.  A sweep takes one time
+// node at a time:
+//   1  g(b) = sum_a P_a(t_k) h(b, a)                     (columns, over the modes b)
+//   2  H on the thread's line of points                  (columns, lines)
+//   3  fluxes F_d at the points, FP64                    (points)
+//   4  each line of F_d projected along x_0, in place    (columns, lines)
+//   5  the projections along the other dimensions, then  acc(b, a) += P_a(t_k) v(b)
+// and after the last node H' = W U - sum_d (Dt/dx_d) C_d acc_d.  Points come
+// in pairs x, -x, so a one-dimensional stage takes half the products.  The
+// first sweep's initial guess does not depend on x_0 (AmrDG.tpp:520-533): its
+// values on the (x_1 .., t) grid are those of U on the spatial grid, so it is
+// one slice whose projections are spread over a_0 with the sums of P_a0.  The
+// mass flux is the momentum, linear in H: its update K_d h comes from the
+// modes, and phases 4 and 5 run over the columns of the other variables.
+//
+// What bounds it: the FP64 pipe (1.6 operations per clock and SM), which now
+// sees the flux evaluations only; the column-per-thread FP64 form of the same
+// sweeps spent three quarters of it on the operators.  The stages are short
+// loops over tables instead of unrolled code per (operator, time node): the
+// integer form issues so much faster that straight-line code starves on
+// instruction fetch (57 k instructions per column, 16 % issue activity).
+#pragma once
+
+#include "adg_kernels.cuh"
+
+namespace adg {
+
+template <class O, int E>
+struct FxShape {
+  static constexpr int D = O::D, Q = O::Q, N = O::N, NP_S = O::NP_S, NP_ST = O::NP_ST, NS = O::NQ_S;
+  static constexpr int C = E * Q;
+  static constexpr int LD = C | 1;  // odd: the point phases read across columns
+  static constexpr int LINES = NS / N;
+  // threads per line: the columns, filled up to whole warps where that idles
+  // few lanes (a warp then works on one line, its table reads are uniform)
+  static constexpr int CP = C % 32 >= 28 ? (C + 31) / 32 * 32 : C;
+  static constexpr int CF = E * (Q - 1);  // columns whose fluxes are projected in the sweeps
+  static constexpr int NT = (CP * LINES + 31) / 32 * 32;
+  static constexpr int ROWS = (NP_ST + LINES - 1) / LINES;            // rows of H_w per thread
+  static constexpr int TASKS = (D * O::FX_NPRE + LINES - 1) / LINES;  // (direction, mode prefix) per thread
+  static constexpr int PTS = (E * NS + NT - 1) / NT;                  // points per thread
+  // warps per SM that the register limit allows: the phases wait at barriers
+  // and on the FP64 pipe, so more blocks beat a few spills (D2P3, 256^2:
+  // 16 / 24 / 32 warps 1330 / 1169 / 1216 us; D3P2, 64^3: 11.9 / 9.0 / 8.5
+  // ms), except where a line is long (D2P6 spills 300 bytes at 24)
+  static constexpr int WARPS = D == 3 ? 32 : N <= 4 ? 24 : 16;
+  static constexpr int MIN_BLOCKS = WARPS * 32 / NT > 0 ? WARPS * 32 / NT : 1;
+  // 64-bit slots: modes, U, g, fluxes, accumulators
+  static constexpr int O_H = 0, O_U = O_H + NP_ST * LD, O_G = O_U + NP_S * LD, O_F = O_G + NP_S * LD,
+                       O_A = O_F + D * NS * LD, SLOTS = O_A + D * NP_ST * LD;
+  // 32-bit words after them, [i][column]: exponents of U, of H, NaN bits,
+  // sum of H; per direction the largest flux so far (high word), the
+  // accumulators' exponent, what the slice raised it by, the largest change
+  static constexpr int I_EU = 0, I_EH = C, I_NAN = 2 * C, I_SUM = 3 * C, I_F = 4 * C, I_EA = I_F + D * C,
+                       I_UP = I_EA + D * C, I_Z = I_UP + D * C, WORDS = I_Z + D * C;
+  static constexpr size_t BYTES = (size_t)SLOTS * 8 + (size_t)WORDS * 4;
+};
+
+// Barrier of a block of NT threads.
+template <int NT>
+__device__ __forceinline__ void fx_sync() {
+  if constexpr (NT == 32)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
+// One-dimensional projection tables: P_a at the nodes, and the corrector's
+// w P_a and w P_a'.
+enum FxTab { FX_P, FX_W, FX_D };
+template <class O, int TAB>
+constexpr int fx_tab_shift() {
+  return TAB == FX_P ? O::FX_SP : TAB == FX_W ? O::FX_SW : O::FX_SD;
+}
+template <class O, int TAB>
+constexpr __host__ __device__ int fx_tab_h(int a, int k) {
+  return TAB == FX_P ? O::fx_ph(a, k) : TAB == FX_W ? O::fx_wh(a, k) : O::fx_dh(a, k);
+}
+template <class O, int TAB>
+constexpr __host__ __device__ int fx_tab_l(int a, int k) {
+  return TAB == FX_P ? O::fx_pl(a, k) : TAB == FX_W ? O::fx_wl(a, k) : O::fx_dl(a, k);
+}
+
+// N line values (with one bit of room) as sums and differences of the pairs.
+template <class O>
+struct FxPairs {
+  static constexpr int J = O::N / 2;
+  long long s[J], d[J], mid;
+  __device__ __forceinline__ explicit FxPairs(const long long* x) {
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      s[j] = x[2 * j] + x[2 * j + 1];
+      d[j] = x[2 * j] - x[2 * j + 1];
+    }
+    mid = O::N % 2 ? x[O::N - 1] : 0;
+  }
+  // row a of the table (a compile-time constant after unrolling)
+  template <int TAB>
+  __device__ __forceinline__ long long row(int a) const {
+    const bool odd = (a % 2 == 1) != (TAB == FX_D);
+    if (TAB == FX_D && a == 0) return 0;
+    if (TAB == FX_P && a == 0 && (O::N & (O::N - 1)) == 0) {  // the factor 2 / N is a shift
+      long long t = J > 1 ? J / 2 : 0;
+#pragma unroll
+      for (int j = 0; j < J; ++j) t += s[j];
+      return J == 1 ? t : J == 2 ? t >> 1 : t >> 2;
+    }
+    FxSum t;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const long long x = odd ? d[j] : s[j];
+      t.mulc(fx_hi(x), fx_lo(x), fx_tab_h<O, TAB>(a, 2 * j), fx_tab_l<O, TAB>(a, 2 * j));
+    }
+    if (O::N % 2 && !odd) t.mulc(fx_hi(mid), fx_lo(mid), fx_tab_h<O, TAB>(a, O::N - 1), fx_tab_l<O, TAB>(a, O::N - 1));
+    return t.get();
+  }
+};
+
+// Modes along x_0 of a line: t(n0) = sum over the other modes of g with the
+// line's values of their Legendre polynomials (c1, and c2 at D = 3; entry 0
+// is one).  g at stride LD.
+template <class O, int LD>
+__device__ __forceinline__ void fx_line_modes(const long long* g, const FxCoef* c1, const FxCoef* c2, long long* t) {
+  constexpr int P = O::P;
+  int b = 0;
+#pragma unroll
+  for (int n0 = 0; n0 <= P; ++n0) {
+    FxSum s;
+#pragma unroll
+    for (int n1 = 0; n1 <= P - n0; ++n1) {
+      long long x;
+      if constexpr (O::D == 2) {
+        x = g[b++ * LD];
+      } else {
+        FxSum r;
+        r.add(g[b++ * LD]);
+#pragma unroll
+        for (int n2 = 1; n2 <= P - n0 - n1; ++n2) r.mul(g[b++ * LD], c2[n2]);
+        x = n0 + n1 < P ? r.get() : r.A;
+      }
+      if (n1 == 0) {
+        s.add(x);
+      } else {
+        if (n1 == 5) s.fold();
+        s.mul(x, c1[n1]);
+      }
+    }
+    t[n0] = n0 < P ? s.get() : s.A;
+  }
+}
+
+// Values at the N points of a line from its modes: out(k0, value).
+template <class O, class Out>
+__device__ __forceinline__ void fx_line_points(const long long* t, Out out) {
+  constexpr int N = O::N, P = O::P;
+  int h[N], l[N];
+#pragma unroll
+  for (int n = 1; n <= P; ++n) {
+    h[n] = fx_hi(t[n]);
+    l[n] = fx_lo(t[n]);
+  }
+#pragma unroll
+  for (int j = 0; j < (N + 1) / 2; ++j) {
+    FxSum ev, od;
+    ev.add(t[0]);
+#pragma unroll
+    for (int n = 1; n <= P; ++n) (n % 2 ? od : ev).mulc(h[n], l[n], O::fx_vh(n, 2 * j), O::fx_vl(n, 2 * j));
+    const long long a = P >= 2 ? ev.get() : ev.A;
+    if (2 * j + 1 < N) {
+      const long long b = od.get();
+      out(2 * j, a + b);
+      out(2 * j + 1, a - b);
+    } else {
+      out(2 * j, a);
+    }
+  }
+}
+
+// Values P_a(x_k) of a line's coordinate k as run-time coefficients.
+template <class O>
+__device__ __forceinline__ void fx_load_coefs(int k, FxCoef* c) {
+#pragma unroll
+  for (int a = 1; a < O::N; ++a) c[a] = O::fx_val(a, k);
+}
+template <class O>
+__device__ __forceinline__ void fx_end_coefs(int side, FxCoef* c) {  // P_a(+-1)
+#pragma unroll
+  for (int a = 1; a < O::N; ++a) c[a] = {a % 2 && !side ? -(1 << kFxLimb) : 1 << kFxLimb, 0};
+}
+
+// The block: what every phase needs, and the thread's column and line, over
+// all columns or over those of the sweeps' flux projections.
+template <class O, int E>
+struct FxBlock {
+  using S = FxShape<O, E>;
+  long long* m;  // shared slots
+  int* w;        // shared words
+  int line, col;
+  bool act;      // the thread has a column
+  __device__ __forceinline__ double* f() const { return reinterpret_cast<double*>(m + S::O_F); }
+  __device__ __forceinline__ int& word(int base, int i = 0) const { return w[base + i * S::C + col]; }
+};
+
+// The largest magnitude (high word) of the thread's line of direction dir's
+// fluxes into the column's.
+template <class O, int E>
+__device__ __forceinline__ void fx_line_max(const FxBlock<O, E>& k, int dir) {
+  using S = FxShape<O, E>;
+  const int* f = reinterpret_cast<const int*>(k.f() + (dir * S::NS + k.line) * S::LD + k.col) + 1;
+  int e = 0;
+#pragma unroll
+  for (int i = 0; i < O::N; ++i) e = max(e, f[i * S::LINES * S::LD * 2] & 0x7fffffff);
+  atomicMax(&k.word(S::I_F, dir), e);
+}
+// The exponent the column's fluxes are read at: one bit of room.
+template <class O, int E>
+__device__ __forceinline__ int fx_line_exp(const FxBlock<O, E>& k, int dir) {
+  return (k.word(FxShape<O, E>::I_F, dir) >> 20) + 1;
+}
+// The line projected along x_0, in the place of its values.
+template <class O, int E, int TAB>
+__device__ __forceinline__ void fx_line_project(const FxBlock<O, E>& k, int dir, int e) {
+  using S = FxShape<O, E>;
+  constexpr int N = O::N;
+  double* f = k.f() + (dir * S::NS + k.line) * S::LD + k.col;
+  long long v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = fx_from_double(f[i * S::LINES * S::LD], e);
+  const FxPairs<O> p(v);
+  long long* t = reinterpret_cast<long long*>(f);
+#pragma unroll
+  for (int a = 0; a < N; ++a) t[a * S::LINES * S::LD] = p.template row<TAB>(a);
+}
+
+// D = 3: projection along x_1 of the values (n0, k1, k2), in place, for the
+// thread's (n0, k2).  Every further dimension halves its operands, one bit of
+// room for the pairs.
+template <class O, int E, int TAB>
+__device__ __forceinline__ void fx_project_planes(const FxBlock<O, E>& k, int dir) {
+  using S = FxShape<O, E>;
+  constexpr int N = O::N, P = O::P;
+  const int n0 = k.line / N, k2 = k.line % N;
+  long long* t = k.m + S::O_F + (dir * S::NS + n0 * S::LINES + k2) * S::LD + k.col;
+  long long v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = fx_half(t[i * N * S::LD]);
+  const FxPairs<O> p(v);
+#pragma unroll
+  for (int a = 0; a < N; ++a)
+    if (a <= P - n0) t[a * N * S::LD] = p.template row<TAB>(a);
+}
+
+// Operands of the last projection of (direction, prefix slot).
+template <class O, int E>
+__device__ __forceinline__ FxPairs<O> fx_last(const FxBlock<O, E>& k, int dir, int slot) {
+  using S = FxShape<O, E>;
+  const long long* t = k.m + S::O_F + (dir * S::NS + slot * O::N) * S::LD + k.col;
+  long long v[O::N];
+#pragma unroll
+  for (int i = 0; i < O::N; ++i) v[i] = fx_half(t[i * S::LD]);
+  return FxPairs<O>(v);
+}
+
+// (direction, prefix) of task j of the thread; false when there is none.
+// Odd directions run through the prefixes backwards, so that a thread's
+// tasks are of both sizes.
+template <class O, int E>
+__device__ __forceinline__ bool fx_task(int line, int j, int* dir, int* pre) {
+  const int i = line + j * FxShape<O, E>::LINES;
+  *dir = i / O::FX_NPRE;
+  *pre = i % O::FX_NPRE;
+  if (*dir & 1) *pre = O::FX_NPRE - 1 - *pre;
+  return i < O::D * O::FX_NPRE;
+}
+
+// Phases 2 to 5 of one slice: H from the spatial modes g (exponent and NaN
+// bits of the column given), fluxes, projections, accumulation.  kt < 0: the
+// first sweep's slice.  k: all columns, kf: those projected.
+template <class O, int E>
+__device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxBlock<O, E>& kf, const long long* g,
+                                               int eg, int nan_bits, const FxCoef* c1, const FxCoef* c2, int kt,
+                                               double gm1) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D, Q = O::Q, N = O::N, P = O::P, LD = S::LD;
+  if (k.act) {
+    long long t[N];
+    fx_line_modes<O, LD>(g + k.col, c1, c2, t);
+    double* h = k.f() + k.line * LD + k.col;
+    fx_line_points<O>(t, [&](int k0, long long v) { h[k0 * S::LINES * LD] = fx_to_double(v, eg, nan_bits); });
+  }
+  fx_sync<S::NT>();
+#pragma unroll
+  for (int r = 0; r < S::PTS; ++r) {
+    const int it = threadIdx.x + r * S::NT;
+    if (it < E * S::NS) {
+      double* base = k.f() + (it % S::NS) * LD + (it / S::NS) * Q;
+      double u[Q], F[D * Q];
+#pragma unroll
+      for (int v = 0; v < Q; ++v) u[v] = base[v];
+      euler_flux_all<D, double>(u, gm1, F);
+#pragma unroll
+      for (int d = 0; d < D; ++d)
+#pragma unroll
+        for (int v = 1; v < Q; ++v) base[d * S::NS * LD + v] = F[d * Q + v];
+    }
+  }
+  fx_sync<S::NT>();
+  if (kf.act) {
+#pragma unroll 1
+    for (int d = 0; d < D; ++d) fx_line_max<O, E>(kf, d);
+  }
+  fx_sync<S::NT>();
+  if (kf.act) {
+#pragma unroll 1
+    for (int d = 0; d < D; ++d) {
+      const int e = fx_line_exp<O, E>(kf, d);
+      if (kf.line == 0) {
+        kf.word(S::I_UP, d) = kt > 0 ? e - kf.word(S::I_EA, d) : 0;
+        kf.word(S::I_EA, d) = e;
+      }
+      fx_line_project<O, E, FX_P>(kf, d, e);
+    }
+  }
+  fx_sync<S::NT>();
+  if constexpr (D == 3) {
+    if (kf.act) {
+#pragma unroll 1
+      for (int d = 0; d < D; ++d) fx_project_planes<O, E, FX_P>(kf, d);
+    }
+    fx_sync<S::NT>();
+  }
+  if (!kf.act) return;
+  FxCoef ct[N];
+#pragma unroll
+  for (int a = 0; a < N; ++a) ct[a] = kt < 0 ? O::fx_ssum(a) : O::fx_valt(a, kt);
+#pragma unroll 1
+  for (int j = 0; j < S::TASKS; ++j) {
+    int d, pre;
+    if (!fx_task<O, E>(kf.line, j, &d, &pre)) continue;
+    const FxPairs<O> p = fx_last<O, E>(kf, d, O::fx_pre_slot(pre));
+    const int deg = O::fx_pre_deg(pre), b0 = O::fx_pre_base(pre);
+    const int up = kf.word(S::I_UP, d);
+    long long* acc = kf.m + S::O_A + d * O::NP_ST * LD + kf.col;
+    long long* q = acc + O::fx_first(b0) * LD;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      if (n > P - deg) break;
+      const long long v = p.template row<FX_P>(n);
+      const int h = fx_hi(v), l = fx_lo(v);
+#pragma unroll
+      for (int a = 0; a < N - n; ++a) {
+        if (a > P - deg - n) break;
+        FxSum s;
+        s.mul(h, l, ct[a].h, ct[a].l);
+        if (kt < 0) {
+          acc[O::fx_init(b0 + n, a) * LD] = s.get();
+        } else {
+          if (kt > 0) s.add(up > 0 ? fx_align(q[a * LD], up) : q[a * LD]);
+          q[a * LD] = s.get();
+        }
+      }
+      q += (P - deg - n + 1) * LD;  // the next mode's
+    }
+  }
+}
+
+// z_d = Dt/dx_d C_d acc_d of the thread's rows; of the mass column K_d times
+// the momentum's modes (first: of the first sweep's initial guess, whose only
+// modes are U's).  One loop over the sparse rows of either.
+template <class O, int E>
+__device__ __forceinline__ void fx_changes(const FxBlock<O, E>& k, const FxFactor* cf, bool first,
+                                           long long (&z)[FxShape<O, E>::ROWS][O::D]) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D;
+  const bool mass = k.col % O::Q == 0;
+  const int nv = mass && first ? O::NP_S : O::NP_ST;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const long long* v = k.m + k.col + (mass ? (first ? S::O_U : S::O_H) + d + 1 : S::O_A + d * O::NP_ST * S::LD);
+    const int table = mass ? D + d : d;
+    int bits = 0;
+#pragma unroll
+    for (int r = 0; r < S::ROWS; ++r) {
+      const int n = k.line + r * S::LINES;
+      z[r][d] = 0;
+      if (n < O::NP_ST) {
+        const int j1 = O::fx_row(table, n + 1);
+        FxSum s;
+#pragma unroll 1
+        for (int j = O::fx_row(table, n), i = 0; j < j1; ++j) {
+          const int c = O::fx_col(j);
+          if (c >= nv) break;
+          s.mul(v[c * S::LD], O::fx_cval(j));
+          if (O::NP_ST > 20 && (++i & 3) == 0) s.fold();
+        }
+        z[r][d] = fx_scale(s.get(), cf[d]);
+        const int hi = (int)(z[r][d] >> 32);
+        bits |= hi ^ (hi >> 31);
+      }
+    }
+    atomicOr(&k.word(S::I_Z, d), bits);
+  }
+}
+
+// H_w' = W U - sum_d z_d: the terms aligned to the largest of U's exponent
+// and the changes' actual ones, then the column rescaled to its sum of
+// magnitudes.
+template <class O, int E>
+__device__ __forceinline__ void fx_update(const FxBlock<O, E>& k, const FxFactor* cf, bool first) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D;
+  long long z[S::ROWS][D];
+  int ez[D], nan_bits = 0, top = 0;
+  if (k.act) {
+    fx_changes<O, E>(k, cf, first, z);
+    const bool mass = k.col % O::Q == 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      if (mass) {
+        const int* w = k.w + k.col + d + 1;  // the momentum's column
+        const int e = first ? w[S::I_EU] : w[S::I_EH];
+        ez[d] = fx_scaled_exp(e, O::fx_sk(d), cf[d]);
+        nan_bits |= first ? 0 : w[S::I_NAN];
+      } else {
+        ez[d] = fx_scaled_exp(k.word(S::I_EA, d), D - 1 + O::fx_sc(d), cf[d]);
+      }
+      nan_bits |= fx_poison(ez[d]);
+    }
+  }
+  fx_sync<S::NT>();
+  if (k.act) {
+    const int eu = k.word(S::I_EU);
+    top = eu;
+    nan_bits |= fx_poison(eu);
+#pragma unroll
+    for (int d = 0; d < D; ++d) top = max(top, ez[d] + 4 - __clz(k.word(S::I_Z, d)));  // |z| < 2^(64 - clz)
+    int sum = 0;
+#pragma unroll
+    for (int r = 0; r < S::ROWS; ++r) {
+      const int n = k.line + r * S::LINES;
+      if (n < O::NP_ST) {
+        long long h = 0;
+        if (O::fx_time(n) == 0) h = fx_align(k.m[S::O_U + O::fx_spatial(n) * S::LD + k.col], top - eu);
+#pragma unroll
+        for (int d = 0; d < D; ++d) h -= fx_move(z[r][d], top - ez[d]);
+        z[r][0] = h;
+        sum += (abs((int)(h >> 32)) >> 6) + 1;  // |h| < 2^38 of these
+      }
+    }
+    atomicAdd(&k.word(S::I_SUM), sum);
+  }
+  fx_sync<S::NT>();
+  if (k.act) {
+    const int up = __clz(k.word(S::I_SUM)) - 10;  // sum |h| < 2^(70 - clz), to be below 2^60
+#pragma unroll
+    for (int r = 0; r < S::ROWS; ++r) {
+      const int n = k.line + r * S::LINES;
+      if (n < O::NP_ST) k.m[S::O_H + n * S::LD + k.col] = fx_move(z[r][0], -up);
+    }
+    if (k.line == 0) {
+      k.word(S::I_EH) = top - up;
+      k.word(S::I_NAN) = nan_bits | fx_poison(top - up);
+#pragma unroll
+      for (int d = 0; d < D; ++d) k.word(S::I_Z, d) = k.word(S::I_F, d) = 0;
+    }
+  }
+  fx_sync<S::NT>();
+}
+
+// The modes b whose g the thread computes: first(b) and degree.
+template <class O, int E>
+struct FxModes {
+  static constexpr int NB = (O::NP_S + FxShape<O, E>::LINES - 1) / FxShape<O, E>::LINES;
+  int first[NB], deg[NB];
+  __device__ __forceinline__ explicit FxModes(const FxBlock<O, E>& k) {
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int b = k.line + i * FxShape<O, E>::LINES;
+      first[i] = b < O::NP_S ? O::fx_first(b) : 0;
+      deg[i] = b < O::NP_S ? O::fx_deg(b) : 0;
+    }
+  }
+};
+// g(b) = sum_a P_a(t_k) h(b, a) of time node kt.
+template <class O, int E>
+__device__ __forceinline__ void fx_time_slice(const FxBlock<O, E>& k, const FxModes<O, E>& md, int kt) {
+  using S = FxShape<O, E>;
+  constexpr int P = O::P;
+  if (k.act) {
+    FxCoef c[O::N];
+    fx_load_coefs<O>(kt, c);
+#pragma unroll
+    for (int i = 0; i < FxModes<O, E>::NB; ++i) {
+      const int b = k.line + i * S::LINES;
+      if (b >= O::NP_S) break;
+      const long long* h = k.m + S::O_H + md.first[i] * S::LD + k.col;
+      FxSum s;
+      s.add(h[0]);
+#pragma unroll
+      for (int a = 1; a <= P; ++a) {
+        if (a > P - md.deg[i]) break;
+        if (a == 5) s.fold();
+        s.mul(h[a * S::LD], c[a]);
+      }
+      k.m[S::O_G + b * S::LD + k.col] = s.get();
+    }
+  }
+  fx_sync<S::NT>();
+}
+
+// Face values of a slice: the two faces of x_0 from the line's modes, the
+// others from lines that run along them (D = 2: the two sides of x_1; D = 3:
+// side and x_2, x_1 and side), written to the trace tiles (time node kt).
+template <class O, int E>
+__device__ __forceinline__ void fx_face_values(const FxBlock<O, E>& k, const long long* t, int eg, int nan_bits,
+                                               double* tr) {
+  constexpr int TT = tr_tile<O>();
+  long long lo = t[0], hi = t[0];
+#pragma unroll
+  for (int n = 1; n <= O::P; ++n) {
+    hi += t[n];
+    lo += n % 2 ? -t[n] : t[n];
+  }
+  tr[k.line] = fx_to_double(lo, eg, nan_bits);
+  tr[TT + k.line] = fx_to_double(hi, eg, nan_bits);
+}
+
+template <class O, int E>
+__device__ __forceinline__ void fx_side_lines(const FxBlock<O, E>& k, const long long* g, int eg, int nan_bits,
+                                              double* tr) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D, N = O::N, TT = tr_tile<O>(), SIDES = D == 2 ? 2 : 4 * N;
+#pragma unroll 1
+  for (int i = k.line; i < SIDES; i += S::LINES) {
+    FxCoef c1[N], c2[N];
+    int face, x;  // face 2d + side, point offset
+    if constexpr (D == 2) {
+      fx_end_coefs<O>(i, c1);
+      face = 2 + i;
+      x = 0;
+    } else {
+      const int side = (i / N) & 1, j = i % N;
+      if (i < 2 * N) {
+        fx_end_coefs<O>(side, c1);
+        fx_load_coefs<O>(j, c2);
+      } else {
+        fx_load_coefs<O>(j, c1);
+        fx_end_coefs<O>(side, c2);
+      }
+      face = (i < 2 * N ? 2 : 4) + side;
+      x = j;
+    }
+    long long t[N];
+    fx_line_modes<O, S::LD>(g + k.col, c1, c2, t);
+    double* out = tr + face * TT + x;
+    fx_line_points<O>(t, [&](int k0, long long v) { out[k0 * (D == 2 ? 1 : N)] = fx_to_double(v, eg, nan_bits); });
+  }
+}
+
+// Corrector volume term of direction DIR from the time-integrated fluxes
+// (AmrDG.tpp:696-709): projections with w P' along DIR and w P along the
+// others; the modes' values as doubles into the accumulators' place.
+template <class O, int E, int DIR>
+__device__ __forceinline__ void fx_volume_last(const FxBlock<O, E>& k, int pre) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D, TAB = DIR == D - 1 ? FX_D : FX_W;
+  const FxPairs<O> p = fx_last<O, E>(k, DIR, O::fx_pre_slot(pre));
+  const int deg = O::fx_pre_deg(pre), ef = fx_line_exp<O, E>(k, DIR);
+  const int e = ef + (D - 1) + O::FX_SD + (D - 1) * O::FX_SW, nan_bits = fx_poison(ef);
+  double* out = reinterpret_cast<double*>(k.m + S::O_A) + (DIR * O::NP_S + O::fx_pre_base(pre)) * S::LD + k.col;
+#pragma unroll
+  for (int n = 0; n < O::N; ++n)
+    if (n <= O::P - deg) out[n * S::LD] = fx_to_double(p.template row<TAB>(n), e, nan_bits);
+}
+
+template <class O, int E>
+__device__ __forceinline__ void fx_volume_term(const FxBlock<O, E>& k) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D;
+  if (k.act) {
+#pragma unroll 1
+    for (int d = 0; d < D; ++d) fx_line_max<O, E>(k, d);
+  }
+  fx_sync<S::NT>();
+  if (k.act) {
+    fx_line_project<O, E, FX_D>(k, 0, fx_line_exp<O, E>(k, 0));
+#pragma unroll 1
+    for (int d = 1; d < D; ++d) fx_line_project<O, E, FX_W>(k, d, fx_line_exp<O, E>(k, d));
+  }
+  fx_sync<S::NT>();
+  if constexpr (D == 3) {
+    if (k.act) {
+      fx_project_planes<O, E, FX_W>(k, 0);
+      fx_project_planes<O, E, FX_D>(k, 1);
+      fx_project_planes<O, E, FX_W>(k, 2);
+    }
+    fx_sync<S::NT>();
+  }
+  if (k.act) {
+#pragma unroll 1
+    for (int j = 0; j < S::TASKS; ++j) {
+      int d, pre;
+      if (!fx_task<O, E>(k.line, j, &d, &pre)) continue;
+      if (d == 0) fx_volume_last<O, E, 0>(k, pre);
+      if (d == 1) fx_volume_last<O, E, 1>(k, pre);
+      if constexpr (D == 3)
+        if (d == 2) fx_volume_last<O, E, 2>(k, pre);
+    }
+  }
+  fx_sync<S::NT>();
+}
+
+// One group of E elements (positions chunk E .. of the range or list).
+template <class O, int E>
+__device__ __forceinline__ void fx_predictor_chunk(const PredictorArgs& a, char* smem, int chunk, int limit) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D, Q = O::Q, N = O::N, NP_S = O::NP_S, NP_ST = O::NP_ST, NS = S::NS, LD = S::LD, C = S::C;
+  constexpr int NB = O::NQ_BD, NSB = NB / N, NF = 2 * D, TT = tr_tile<O>(), NT = S::NT;
+  FxBlock<O, E> k;
+  k.m = reinterpret_cast<long long*>(smem);
+  k.w = reinterpret_cast<int*>(k.m + S::SLOTS);
+  k.line = threadIdx.x / S::CP;
+  k.act = k.line < S::LINES && (int)threadIdx.x % S::CP < C;
+  k.col = k.act ? threadIdx.x % S::CP : 0;
+  FxBlock<O, E> kf = k;  // the columns of the sweeps' flux projections: all but the mass
+  kf.line = threadIdx.x / S::CF;
+  kf.col = (threadIdx.x % S::CF) / (Q - 1) * Q + 1 + (threadIdx.x % S::CF) % (Q - 1);
+  kf.act = kf.line < S::LINES;
+  const int e0 = chunk * E;
+  auto element = [&](int el) {  // past the end: the last one (its results are not written)
+    const int i = e0 + el < limit ? e0 + el : limit - 1;
+    return a.elem_list ? a.elem_list[i] : i;
+  };
+  const int el = k.col / Q, q = k.col % Q;
+  const bool live = e0 + el < limit;
+  const int e = element(el);
+  const int lev = a.elem_level ? a.elem_level[e] : 0;
+  double c[D];
+  FxFactor cf[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    c[d] = a.dt[kScalDtDx + 3 * lev + d];
+    cf[d] = fx_factor(c[d]);
+  }
+  const double gm1 = a.gamma - 1.0;
+  const FxModes<O, E> md(k);
+  FxCoef c1[N], c2[N];
+  fx_load_coefs<O>(D == 2 ? k.line % N : (k.line / N) % N, c1);
+  if constexpr (D == 3) fx_load_coefs<O>(k.line % N, c2);
+
+  // U: coalesced loads, the column's exponent, fixed point
+  double* ud = reinterpret_cast<double*>(k.m + S::O_G);
+  for (int i = threadIdx.x; i < C * NP_S; i += NT)
+    ud[(i % NP_S) * LD + i / NP_S] = a.Uw[(size_t)element(i / (Q * NP_S)) * Q * NP_S + i % (Q * NP_S)];
+  fx_sync<S::NT>();
+  if (k.act && k.line == 0) {
+    const int eu = fx_norm_exp<NP_S>(ud + k.col, LD);
+    k.word(S::I_EU) = eu;
+    k.word(S::I_SUM) = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) k.word(S::I_Z, d) = k.word(S::I_F, d) = 0;
+    if (a.ubar_old && live) a.ubar_old[(size_t)e * Q + q] = ud[k.col];
+  }
+  fx_sync<S::NT>();
+  if (k.act)
+    for (int b = k.line; b < NP_S; b += S::LINES)
+      k.m[S::O_U + b * LD + k.col] = fx_from_double(ud[b * LD + k.col], k.word(S::I_EU));
+  fx_sync<S::NT>();
+
+  // the first sweep on U, then the others (AmrDG.h:1103-1119)
+  {
+    const int eu = k.act ? k.word(S::I_EU) : 0;
+    fx_sweep_slice<O, E>(k, kf, k.m + S::O_U, eu, fx_poison(eu), c1, c2, -1, gm1);
+    fx_sync<S::NT>();
+    fx_update<O, E>(k, cf, true);
+  }
+#pragma unroll 1
+  for (int s = 1; s < a.sweeps; ++s) {
+    if (k.act && k.line == 0) k.word(S::I_SUM) = 0;
+    const int eh = k.act ? k.word(S::I_EH) : 0, nan_bits = k.act ? k.word(S::I_NAN) : 0;
+#pragma unroll 1
+    for (int kt = 0; kt < N; ++kt) {
+      fx_time_slice<O, E>(k, md, kt);
+      fx_sweep_slice<O, E>(k, kf, k.m + S::O_G, eh, nan_bits, c1, c2, kt, gm1);
+    }
+    fx_sync<S::NT>();
+    fx_update<O, E>(k, cf, false);
+  }
+  const int eh = k.act ? k.word(S::I_EH) : 0, nan_bits = k.act ? k.word(S::I_NAN) : 0;
+  if (a.Hw_out && k.act && live) {
+    double* dst = a.Hw_out + ((size_t)e * Q + q) * NP_ST;
+    for (int n = k.line; n < NP_ST; n += S::LINES) {
+      bool same = true;
+      for (int t = 0; t < D; ++t) same = same && O::fx_row(t, n) == O::fx_row(t, n + 1);
+      dst[n] = fx_to_double(k.m[S::O_H + n * LD + k.col], eh, nan_bits);
+      // a mode that no sweep changes is U's own
+      if (same) dst[n] = O::fx_time(n) == 0 ? a.Uw[((size_t)e * Q + q) * NP_S + O::fx_spatial(n)] : 0.0;
+    }
+  }
+
+  // final stage: per time node the face values and the volume fluxes, these
+  // integrated over time by the threads of the points
+  double fbar[S::PTS][D * Q];
+#pragma unroll
+  for (int r = 0; r < S::PTS; ++r)
+#pragma unroll
+    for (int v = 0; v < D * Q; ++v) fbar[r][v] = 0.0;
+#pragma unroll 1
+  for (int kt = 0; kt < N; ++kt) {
+    fx_time_slice<O, E>(k, md, kt);
+    if (k.act) {
+      const long long* g = k.m + S::O_G;
+      long long t[N];
+      fx_line_modes<O, LD>(g + k.col, c1, c2, t);
+      double* h = k.f() + k.line * LD + k.col;
+      fx_line_points<O>(t, [&](int k0, long long v) { h[k0 * S::LINES * LD] = fx_to_double(v, eh, nan_bits); });
+      if (live) {
+        double* tr = a.Tr + (size_t)e * NF * TT + q * NB + kt * NSB;
+        fx_face_values<O, E>(k, t, eh, nan_bits, tr);
+        fx_side_lines<O, E>(k, g, eh, nan_bits, tr);
+      }
+    }
+    fx_sync<S::NT>();
+    const double w = O::weight(kt);
+#pragma unroll
+    for (int r = 0; r < S::PTS; ++r) {
+      const int it = threadIdx.x + r * NT;
+      if (it < E * NS) {
+        const double* base = k.f() + (it % NS) * LD + (it / NS) * Q;
+        double u[Q], F[D * Q];
+#pragma unroll
+        for (int v = 0; v < Q; ++v) u[v] = base[v];
+        euler_flux_all<D, double>(u, gm1, F);
+#pragma unroll
+        for (int v = 0; v < D * Q; ++v) fbar[r][v] = fma(w, F[v], fbar[r][v]);
+      }
+    }
+  }
+  fx_sync<S::NT>();
+#pragma unroll
+  for (int r = 0; r < S::PTS; ++r) {
+    const int it = threadIdx.x + r * NT;
+    if (it < E * NS) {
+      double* base = k.f() + (it % NS) * LD + (it / NS) * Q;
+#pragma unroll
+      for (int d = 0; d < D; ++d)
+#pragma unroll
+        for (int v = 0; v < Q; ++v) base[d * NS * LD + v] = fbar[r][d * Q + v];
+    }
+  }
+  fx_sync<S::NT>();
+  fx_volume_term<O, E>(k);
+  // Rvol = M U + sum_d (Dt/dx_d) Sk_d F_d, coalesced
+  const double* vt = reinterpret_cast<const double*>(k.m + S::O_A);
+  for (int i = threadIdx.x; i < C * NP_S; i += NT) {
+    const int b = i % NP_S, cc = i / NP_S;
+    if (e0 + cc / Q >= limit) continue;
+    const size_t o = (size_t)element(cc / Q) * Q * NP_S + i % (Q * NP_S);
+    const int lv = a.elem_level ? a.elem_level[element(cc / Q)] : 0;
+    double r = O::mdiag(b) * a.Uw[o];
+#pragma unroll
+    for (int d = 0; d < D; ++d) r = fma(a.dt[kScalDtDx + 3 * lv + d], vt[(d * NP_S + b) * LD + cc], r);
+    a.Rvol[o] = r;
+  }
+  // face physics (AmrDG.h:1207-1251) on the values in the trace tiles
+  for (int it = threadIdx.x; it < E * NF * NB; it += NT) {
+    const int p = it % NB, face = (it / NB) % NF, ee = it / (NB * NF);
+    if (e0 + ee >= limit) break;
+    double* t = a.Tr + ((size_t)element(ee) * NF + face) * TT + p;
+    double uu[Q], F[Q];
+#pragma unroll
+    for (int v = 0; v < Q; ++v) uu[v] = t[v * NB];
+    const double df = euler_flux_normal<D>(face >> 1, uu, a.gamma, F);
+#pragma unroll
+    for (int v = 0; v < Q; ++v) t[(Q + v) * NB] = F[v];
+    t[2 * Q * NB] = df;
+  }
+}
+
+template <class O, int E>
+__global__ void __launch_bounds__((FxShape<O, E>::NT), (FxShape<O, E>::MIN_BLOCKS)) k_predictor_fx(PredictorArgs a) {
+  extern __shared__ __align__(16) char fx_smem[];
+  fx_predictor_chunk<O, E>(a, fx_smem, blockIdx.x, a.n_elem);
+}
+
+// The fallback pass: a short grid striding over a list counted on the device.
+template <class O, int E>
+__global__ void __launch_bounds__((FxShape<O, E>::NT)) k_predictor_fx_list(PredictorArgs a) {
+  extern __shared__ __align__(16) char fx_smem[];
+  const int limit = *a.list_count;
+  if (a.count_total && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(a.count_total, (unsigned long long)limit);
+#pragma unroll 1
+  for (int chunk = blockIdx.x; chunk * E < limit; chunk += gridDim.x) {
+    fx_predictor_chunk<O, E>(a, fx_smem, chunk, limit);
+    fx_sync<FxShape<O, E>::NT>();
+  }
+}
+
+}  // namespace adg

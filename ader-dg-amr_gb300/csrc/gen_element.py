@@ -208,7 +208,7 @@ class Element:
         Vf = [[fr(v) for v in r] for r in V]
         G = mat_mul(transpose(Vf), Vf)
         Ginv = mat_inv(G)
-        self.Ginv = Ginv
+        self.G, self.Ginv = G, Ginv
         Vinv = mat_mul(Ginv, transpose(Vf))
         # Mk_h_w, Mk_pred, Sk_pred (exact)
         Mkhw = [[Fraction(0)] * nst for _ in range(nst)]
@@ -767,6 +767,146 @@ def emit_op(name, op):
     return "\n".join(lines), nops
 
 
+# ----------------------------------------------------------------------------
+# Fixed-point tables of the plain predictor (adg_fx.cuh): one-dimensional
+# Legendre tables and the sparse C_d as limbs of 60-bit fractions.
+# ----------------------------------------------------------------------------
+FX_FRAC, FX_LIMB = 60, 30
+
+
+def fx_limbs(coef, s):
+    """Limbs (high, signed low) of coef 2^-s."""
+    c = Fraction(coef) * Fraction(2) ** (FX_FRAC - s)
+    n = math.floor(c + Fraction(1, 2))
+    lo = ((n + (1 << (FX_LIMB - 1))) & ((1 << FX_LIMB) - 1)) - (1 << (FX_LIMB - 1))
+    hi = (n - lo) >> FX_LIMB
+    assert abs(hi) <= 1 << (FX_FRAC - FX_LIMB)
+    return hi, lo
+
+
+def emit_fx(el, ops):
+    """(tables at namespace scope, members of Ops).  A projection pairs the
+    points x and -x first, with one bit of room, and its coefficients are
+    divided by the largest row sum over the pairs, so that the sums keep the
+    operands' bound: exponent + 1 per dimension.  The factors the projections
+    lose that way ((N/2)^D, and N over the time slices) are put back into C_d,
+    the corrector's into its tables' powers of two."""
+    import numpy as np
+
+    D, P, N = el.D, el.P, el.N
+    tabs = {"v": [[el.val[a][k] for k in range(N)] for a in range(N)],
+            "p": [[Fraction(el.val[a][k]) * 2 / N for k in range(N)] for a in range(N)],
+            "w": [[el.val[a][k] * el.weights[k] for k in range(N)] for a in range(N)],
+            "d": [[el.dval[a][k] * el.weights[k] for k in range(N)] for a in range(N)]}
+    scale = {"v": 0, "p": 0}
+    for t in "wd":
+        m = max(sum(abs(c) for c in row) for row in tabs[t]) / 2
+        big = max(abs(c) for row in tabs[t] for c in row)
+        scale[t] = max(0, math.ceil(math.log2(max(m, big)) - 1e-9))
+    for a in range(N):  # parity of the tables, which the pairing relies on
+        for j in range(N // 2):
+            assert el.val[a][2 * j + 1] == (-1) ** a * el.val[a][2 * j] and el.weights[2 * j] == el.weights[2 * j + 1]
+            assert el.dval[a][2 * j + 1] == -(-1) ** a * el.dval[a][2 * j]
+
+    def select(vals):
+        expr = str(vals[-1])
+        for i in range(len(vals) - 2, -1, -1):
+            expr = f"i == {i} ? {vals[i]} : ({expr})"
+        return expr
+    head, mem = [], []
+    for t, rows in tabs.items():
+        lim = [fx_limbs(c, scale[t]) for row in rows for c in row]
+        for part, name in ((0, "h"), (1, "l")):
+            mem.append(f"  static constexpr __host__ __device__ int fx_{t}{name}(int a, int k) {{ const int i = a * {N} + k; "
+                       f"return {select([x[part] for x in lim])}; }}")
+        mem.append(f"  static constexpr int FX_S{t.upper()} = {scale[t]};")
+
+    def ints(name, vals, typ="int"):
+        head.append(f"__device__ __constant__ const {typ} {name}[] = {{" + ", ".join(str(v) for v in vals) + "};")
+
+    def coefs(name, lim):
+        head.append(f"__device__ __constant__ const FxCoef {name}[] = {{" + ", ".join("{%d, %d}" % x for x in lim) + "};")
+    # val[a][k] at run-time indices: plain, and over N; the sums of a row over
+    # N, which the x_0-independent first sweep's fluxes are multiplied by
+    coefs("FX_VAL_", [fx_limbs(el.val[a][k], 0) for a in range(N) for k in range(N)])
+    coefs("FX_VALT_", [fx_limbs(Fraction(el.val[a][k]) / N, 0) for a in range(N) for k in range(N)])
+    ssum = [sum(Fraction(el.val[a][k]) for k in range(N)) if a % 2 == 0 else Fraction(0) for a in range(N)]
+    coefs("FX_SSUM_", [fx_limbs(v / N if abs(v) > 1e-13 else 0, 0) for v in ssum])
+    # space-time mode of (spatial mode b, time degree a) is first(b) + a; of
+    # (degree a_0, modes b of the remaining dimensions) it is listed
+    pos = {n: i for i, n in enumerate(el.mi_st)}
+    ints("FX_DEG_", [sum(b) for b in el.mi_s], "signed char")
+    ints("FX_FIRST_", [pos[b + (0,)] for b in el.mi_s], "short")  # then (b, a) is FIRST + a
+    for b in el.mi_s:
+        assert all(pos[b + (a,)] == pos[b + (0,)] + a for a in range(P - sum(b) + 1))
+    ints("FX_INIT_", [pos.get((a,) + b, 0) for b in el.mi_s for a in range(N)], "short")
+    ints("FX_SPATIAL_", el.st_space, "short")
+    ints("FX_TIME_", el.st_time, "signed char")
+    # mode prefixes (all dimensions but the last): their slot among the N^(D-1)
+    # tensor indices, first spatial mode and degree
+    pre = [m for m in itertools.product(range(N), repeat=D - 1) if sum(m) <= P]
+    ints("FX_PRE_SLOT_", [sum(k * N ** (D - 2 - i) for i, k in enumerate(m)) for m in pre], "short")
+    ints("FX_PRE_BASE_", [el.mi_s.index(m + (0,)) for m in pre], "short")
+    ints("FX_PRE_DEG_", [sum(m) for m in pre], "signed char")
+    mem.append(f"  static constexpr int FX_NPRE = {len(pre)};")
+    # C_d: sparse rows, scaled by the bound of A_d F over the operands' growth;
+    # K_d = C_d V^T V, the same update of a flux that is linear in H (the mass
+    # flux is the momentum), from H's modes
+    lost = Fraction(N, 2) ** D * N
+    KS = []
+    for d in range(D):
+        Cf = [[Fraction(0)] * el.Np_st for _ in range(el.Np_st)]
+        for r, row in enumerate(ops[f"cproj{d}"][0][0].rows):
+            for c, v in row:
+                Cf[r][c] = Fraction(v)
+        K = to_float(mat_mul(Cf, el.G))
+        big = max(abs(v) for r in K for v in r)
+        KS.append([[(c, v) for c, v in enumerate(r) if abs(v) > 1e-11 * big] for r in K])
+    shifts, kshifts, sparse = [], [], []
+    for d in range(D):
+        stages = ops[f"cproj{d}"][0]
+        assert len(stages) == 1
+        rows = [[(c, Fraction(v) * lost) for c, v in r] for r in stages[0].rows]
+        m = np.abs(np.array(el.A[d])).sum(axis=1).max()
+        big = float(max(abs(v) for r in rows for _, v in r))
+        shifts.append(max(math.ceil(math.log2(m) - 1e-9) - D, math.ceil(math.log2(big) - 1e-9)))
+        kshifts.append(math.ceil(math.log2(max(abs(v) for r in KS[d] for _, v in r)) - 1e-9))
+        sparse.append((rows, shifts[d]))
+    sparse += [(KS[d], kshifts[d]) for d in range(D)]
+    # (short rows are summed without folding the middle products in between)
+    assert el.Np_st > 20 or max(len(r) for rr, _ in sparse for r in rr) <= 5
+    # one table of rows: C_0 .. C_{D-1}, K_0 .. K_{D-1}
+    off, col, lim = [], [], []
+    for rr, sh in sparse:
+        off.append(len(col))
+        for r in rr:
+            for c, v in r:
+                col.append(c)
+                lim.append(fx_limbs(v, sh))
+            off.append(len(col))
+    ints("FX_ROW_", off, "short")
+    ints("FX_COL_", col, "short")
+    coefs("FX_CVAL_", lim)
+    mem.append("  static constexpr __host__ __device__ int fx_sk(int d) { return "
+               + "".join(f"d == {d} ? {s} : " for d, s in enumerate(kshifts[:-1])) + f"{kshifts[-1]}; }}")
+    mem.append("  static constexpr __host__ __device__ int fx_sc(int d) { return "
+               + "".join(f"d == {d} ? {s} : " for d, s in enumerate(shifts[:-1])) + f"{shifts[-1]}; }}")
+    for name, typ, args in (("val", "FxCoef", "int a, int k"), ("valt", "FxCoef", "int a, int k")):
+        mem.append(f"  static __device__ __forceinline__ FxCoef fx_{name}({args}) {{ return FX_{name.upper()}_[a * {N} + k]; }}")
+    mem.append("  static __device__ __forceinline__ FxCoef fx_ssum(int a) { return FX_SSUM_[a]; }")
+    mem.append("  static __device__ __forceinline__ int fx_deg(int b) { return FX_DEG_[b]; }")
+    mem.append("  static __device__ __forceinline__ int fx_first(int b) { return FX_FIRST_[b]; }")
+    mem.append(f"  static __device__ __forceinline__ int fx_init(int b, int a) {{ return FX_INIT_[b * {N} + a]; }}")
+    mem.append("  static __device__ __forceinline__ int fx_spatial(int n) { return FX_SPATIAL_[n]; }")
+    mem.append("  static __device__ __forceinline__ int fx_time(int n) { return FX_TIME_[n]; }")
+    for k in ("slot", "base", "deg"):
+        mem.append(f"  static __device__ __forceinline__ int fx_pre_{k}(int i) {{ return FX_PRE_{k.upper()}_[i]; }}")
+    mem.append(f"  static __device__ __forceinline__ int fx_row(int t, int n) {{ return FX_ROW_[t * {el.Np_st + 1} + n]; }}")
+    mem.append("  static __device__ __forceinline__ int fx_col(int j) { return FX_COL_[j]; }")
+    mem.append("  static __device__ __forceinline__ FxCoef fx_cval(int j) { return FX_CVAL_[j]; }")
+    return head, mem
+
+
 def add_ic_proj(el, ops):
     """quadmat (AmrDG_ElementMatrix.tpp:154-168): spatial points -> spatial modes."""
     D, P, N = el.D, el.P, el.N
@@ -1049,6 +1189,7 @@ def generate(D, P, out_path):
     add_amr_ops(el, ops)
     n_mom = add_face_moment_ops(el, ops)
     zero_ops = denoise(ops)
+    fx_head, fx_members = emit_fx(el, ops)
     N = P + 1
     qst = N ** (D + 1)
     qbd = N ** D
@@ -1063,6 +1204,7 @@ def generate(D, P, out_path):
         "__device__ __constant__ const double NODES_[] = {" + ", ".join(lit(v) for v in el.nodes) + "};",
         "__device__ __constant__ const double WEIGHTS_[] = {" + ", ".join(lit(v) for v in el.weights) + "};",
         "__device__ __constant__ const float WEIGHTS_F_[] = {" + ", ".join(lit(v) for v in el.weights) + "};",
+        *fx_head,
         "struct Ops {",
         f"  static constexpr int D = {D};",
         f"  static constexpr int P = {P};",
@@ -1167,6 +1309,7 @@ def generate(D, P, out_path):
                         if mi[d] == 1 and all(mi[a] == 0 for a in range(D) if a != d)))
     hdr.append("  static __device__ __forceinline__ int lin_mode(int d) { return "
                + " : ".join(f"d == {d} ? {lin[d]}" for d in range(D - 1)) + f" : {lin[D - 1]}; }}")
+    hdr += fx_members
     hdr.append("};")
     hdr.append("}}  // namespace")
     hdr.append("")

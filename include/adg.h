@@ -443,7 +443,8 @@ int adg_ader_step_noalloc(int D, int P, const int n_cell[3], const double prob_l
                           double gamma, double dt, double* U_w, void* stream);
 
 /* Algorithmic FP64 flops per element-step (the method's dense matvec count)
- * and the FP64 operations the generated kernels actually issue per element. */
+ * and the FP64 operations of its factorised linear stages per element (the
+ * plain predictor runs these in fixed point). */
 int adg_flops_per_element(int D, int P, double* algorithmic, double* issued);
 
 #ifdef __cplusplus
