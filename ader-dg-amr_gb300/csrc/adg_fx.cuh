@@ -111,7 +111,8 @@ __device__ __forceinline__ long long fx_half(long long v) { return (v + 1) >> 1;
 __device__ __forceinline__ long long fx_align(long long v, int shift) { return v >> (shift < 63 ? shift : 63); }
 // the same for a shift of either sign
 __device__ __forceinline__ long long fx_move(long long v, int shift) {
-  return fx_align(v << (shift < 0 ? -shift : 0), shift > 0 ? shift : 0);
+  if (shift <= 0) return v << -shift;
+  return fx_align(v, shift);
 }
 
 // A positive double as a 60-bit fraction times 2^(ef - 1022).
@@ -136,6 +137,29 @@ __device__ __forceinline__ int fx_scaled_exp(int e, int growth, const FxFactor& 
   return e > kFxMaxExp || f.ef == 2047 ? kFxNanExp : e + growth + f.ef - 1022;
 }
 
+// Product of two column values: exponents add, less 1022.
+__device__ __forceinline__ long long fx_mul(int ah, int al, int bh, int bl) {
+  FxSum s;
+  s.mul(ah, al, bh, bl);
+  return s.get();
+}
+
+// Reciprocal of v, 2^40 <= v < 2^60, n = clz(v): 2^(123 - n) / v, in
+// (2^59, 2^60].  The FP32 estimate r of the significand x in [1, 2) (24
+// bits), e = 1 - x r exactly, one third-order Householder step r (1 + e + e^2).
+__device__ __forceinline__ long long fx_reciprocal(long long v, int n) {
+  const unsigned long long x = (unsigned long long)v << (n - 4);  // [2^59, 2^60)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;"
+      : "=f"(r)
+      : "f"(__int_as_float(0x3f800000 | (((int)(x >> 36)) & 0x7fffff))));
+  const unsigned r0 = (unsigned)__float2int_rn(r * 16777216.0f);  // 2^24 r, exact
+  const long long e = -(long long)(x * r0);                       // 2^83 e: the product's 2^83 leaves 64 bits
+  const int eh = (int)(e >> 32);
+  const long long p = (e >> 23) + (((long long)eh * eh) >> 42);   // 2^60 (e + e^2)
+  return ((long long)r0 << 36) + (((long long)r0 * p) >> 24);
+}
+
 // Exponent E with sum |x_n| <= 2^(E - 1022), x_n at stride s: the largest
 // exponent field plus what the sum of the truncated significands (20 bits,
 // rounded up) needs.  2047 (infinity or NaN) stays above kFxMaxExp.
@@ -153,6 +177,109 @@ __device__ __forceinline__ int fx_norm_exp(const double* x, int s) {
   }
   const int bits = 32 - __clz(sum);  // sum < 2^bits, in units of 2^(top - 1023 - 20)
   return top + (bits > 21 ? bits - 21 : 0);
+}
+
+// ---------------------------------------------------------------------------
+// The Euler fluxes of a point (Compressible_Euler.h:370-487, 562-589) on
+// column values.  A 60-bit product is about 10 integer instructions, a third
+// of what one FP64 operation keeps its pipe busy for; the exponents of all
+// intermediate values are the element's, so a point does no normalisation
+// but the density's.
+// ---------------------------------------------------------------------------
+
+// Exponents: em momenta, ee energy, er density; n: the largest number of
+// leading zeros of the element's densities, which bounds 1 / rho; gef: that
+// of gamma - 1 (FxFactor::ef).
+template <int D>
+struct FxFluxExp {
+  int xv[D];  // velocities
+  int xk[D];  // m_d v_d
+  int xp, xe, xd[D];
+  __device__ __forceinline__ FxFluxExp(const int* em, int ee, int er, int n, int gef) {
+    int top = ee;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      xv[d] = em[d] + n - er + 1019;
+      xk[d] = xv[d] + em[d] - 1022;
+      top = max(top, xk[d]);
+    }
+    xp = top + 1 + gef - 1022;
+    xe = max(ee, xp) + 1;
+#pragma unroll
+    for (int d = 0; d < D; ++d) xd[d] = max(xk[d], xp) + 1;
+  }
+  // exponent of flux d of variable q >= 1
+  __device__ __forceinline__ int flux(int d, int q, const int* em) const {
+    int x = xe + xv[0] - 1022, o = xd[0];
+#pragma unroll
+    for (int k = 0; k < D; ++k)
+      if (k == d) {
+        x = xe + xv[k] - 1022;
+        o = xd[k];
+      }
+    if (q == D + 1) return x;
+    if (q == d + 1) return o;
+    int v = xv[0], m = em[0];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      if (k == d) v = xv[k];
+      if (k == q - 1) m = em[k];
+    }
+    return v + m - 1022;
+  }
+};
+
+// Smallest density the integer path takes (2^-20 of its bound), and the most
+// the densities of an element may lie apart (as a power of two).
+constexpr long long kFxMinRho = 1LL << 40;
+constexpr int kFxRhoSpan = 6;
+
+// Fluxes F[d][q - 1], q >= 1, at exponents x.flux(d, q).  False where the
+// density is out of range or the pressure within 2^-40 of its terms (or at
+// the floor): such points are for the FP64 evaluation.
+template <int D>
+__device__ __forceinline__ bool fx_euler_flux(const long long* u, const FxFluxExp<D>& x, int ee, int n_max,
+                                              const FxFactor& gm1, long long (&F)[D][D + 1]) {
+  if (u[0] < kFxMinRho || u[0] >= (1LL << 60)) return false;
+  const int n = __clz((int)(u[0] >> 32));
+  if (n_max - n > kFxRhoSpan) return false;
+  const long long r = fx_reciprocal(u[0], n) >> (n_max - n);
+  const int rh = fx_hi(r), rl = fx_lo(r);
+  int mh[D], ml[D], vh[D], vl[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    mh[d] = fx_hi(u[d + 1]);
+    ml[d] = fx_lo(u[d + 1]);
+    const long long v = fx_mul(mh[d], ml[d], rh, rl);
+    vh[d] = fx_hi(v);
+    vl[d] = fx_lo(v);
+  }
+  const int top = x.xp - gm1.ef + 1022;
+  long long p = fx_align(u[D + 1], top - ee);
+  long long w[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    w[d] = fx_mul(mh[d], ml[d], vh[d], vl[d]);
+    p -= fx_align(w[d], top - x.xk[d] + 1);
+  }
+  p = fx_scale(p, gm1);
+  if (p < (1LL << 20)) return false;
+  const long long ep = fx_align(u[D + 1], x.xe - ee) + fx_align(p, x.xe - x.xp);
+  const int eh = fx_hi(ep), el = fx_lo(ep);
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      if (k < d)
+        F[d][k] = F[k][d];  // m_k v_d = m_d v_k
+      else if (k == d)
+        F[d][k] = fx_align(w[d], x.xd[d] - x.xk[d]) + fx_align(p, x.xd[d] - x.xp);
+      else
+        F[d][k] = fx_mul(mh[k], ml[k], vh[d], vl[d]);
+    }
+    F[d][D] = fx_mul(eh, el, vh[d], vl[d]);
+  }
+  return true;
 }
 
 }  // namespace adg

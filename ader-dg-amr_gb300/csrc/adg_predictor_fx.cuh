@@ -1,12 +1,12 @@
-// Plain Picard predictor (AmrDG.tpp:495-537, 744-827) with its linear
-// operators in fixed point (adg_fx.cuh) and its fluxes in FP64.
+// Plain Picard predictor (AmrDG.tpp:495-537, 744-827) in fixed point
+// (adg_fx.cuh); FP64 is left to the final stage's fluxes and the face physics.
 //
 // A block holds E elements, C = E Q columns, and gives every column
 // N^(D-1) threads, one per line of points along x_0.  A sweep takes one time
 // node at a time:
 //   1  g(b) = sum_a P_a(t_k) h(b, a)                     (columns, over the modes b)
 //   2  H on the thread's line of points                  (columns, lines)
-//   3  fluxes F_d at the points, FP64                    (points)
+//   3  fluxes F_d at the points                          (points)
 //   4  each line of F_d projected along x_0, in place    (columns, lines)
 //   5  the projections along the other dimensions, then  acc(b, a) += P_a(t_k) v(b)
 // and after the last node H' = W U - sum_d (Dt/dx_d) C_d acc_d.  Points come
@@ -17,12 +17,21 @@
 // mass flux is the momentum, linear in H: its update K_d h comes from the
 // modes, and phases 4 and 5 run over the columns of the other variables.
 //
-// What bounds it: the FP64 pipe (1.6 operations per clock and SM), which now
-// sees the flux evaluations only; the column-per-thread FP64 form of the same
-// sweeps spent three quarters of it on the operators.  The stages are short
-// loops over tables instead of unrolled code per (operator, time node): the
-// integer form issues so much faster that straight-line code starves on
-// instruction fetch (57 k instructions per column, 16 % issue activity).
+// Phase 3 evaluates the fluxes on the column values (fx_euler_flux); an
+// element with a point whose density or pressure is out of that form's range
+// (near vacuum, at the pressure floor, densities more than 2^6 apart) takes
+// the FP64 fluxes for all of its points, and so do values that are not finite.
+//
+// Why this form: GB300 issues 1.6 FP64 operations per clock and SM.  The
+// column-per-thread FP64 predictor kept that pipe 84 % busy; with the
+// operators on the integer pipes it still set the time through the fluxes
+// (D2P3, 256^2: 2330 -> 1169 us), and with integer fluxes in the sweeps the
+// kernel issues 2.0 instructions per clock and SM (1169 -> 1000 us; a flux
+// costs the integer pipes what its conversions cost before).  Now: dependent
+// integer chains and the barriers between phases.  The stages are short loops
+// over tables instead of unrolled code per (operator, time node):
+// straight-line code starved on instruction fetch (57 k instructions per
+// column, 16 % issue activity).
 #pragma once
 
 #include "adg_kernels.cuh"
@@ -53,10 +62,13 @@ struct FxShape {
   static constexpr int O_H = 0, O_U = O_H + NP_ST * LD, O_G = O_U + NP_S * LD, O_F = O_G + NP_S * LD,
                        O_A = O_F + D * NS * LD, SLOTS = O_A + D * NP_ST * LD;
   // 32-bit words after them, [i][column]: exponents of U, of H, NaN bits,
-  // sum of H; per direction the largest flux so far (high word), the
-  // accumulators' exponent, what the slice raised it by, the largest change
-  static constexpr int I_EU = 0, I_EH = C, I_NAN = 2 * C, I_SUM = 3 * C, I_F = 4 * C, I_EA = I_F + D * C,
-                       I_UP = I_EA + D * C, I_Z = I_UP + D * C, WORDS = I_Z + D * C;
+  // sum of H; in the mass columns the most leading zeros of the slice's
+  // densities, and whether the element's fluxes are FP64; per direction the
+  // exponent of the slice's fluxes, that of the largest so far, the
+  // accumulators', what the slice raised it by, the largest change
+  static constexpr int I_EU = 0, I_EH = C, I_NAN = 2 * C, I_SUM = 3 * C, I_N = 4 * C, I_F64 = 5 * C, I_X = 6 * C,
+                       I_F = I_X + D * C, I_EA = I_F + D * C, I_UP = I_EA + D * C, I_Z = I_UP + D * C,
+                       WORDS = I_Z + D * C;
   static constexpr size_t BYTES = (size_t)SLOTS * 8 + (size_t)WORDS * 4;
 };
 
@@ -205,33 +217,48 @@ struct FxBlock {
   __device__ __forceinline__ int& word(int base, int i = 0) const { return w[base + i * S::C + col]; }
 };
 
-// The largest magnitude (high word) of the thread's line of direction dir's
-// fluxes into the column's.
+constexpr int kFxNoExp = -30000;  // below every exponent
+
+// The exponent of the largest magnitude on the thread's line of direction
+// dir's fluxes into the column's: doubles, or column values of exponent x.
 template <class O, int E>
-__device__ __forceinline__ void fx_line_max(const FxBlock<O, E>& k, int dir) {
+__device__ __forceinline__ void fx_line_max(const FxBlock<O, E>& k, int dir, bool f64, int x) {
   using S = FxShape<O, E>;
   const int* f = reinterpret_cast<const int*>(k.f() + (dir * S::NS + k.line) * S::LD + k.col) + 1;
-  int e = 0;
+  int e = 0, bits = 0;
 #pragma unroll
-  for (int i = 0; i < O::N; ++i) e = max(e, f[i * S::LINES * S::LD * 2] & 0x7fffffff);
-  atomicMax(&k.word(S::I_F, dir), e);
+  for (int i = 0; i < O::N; ++i) {
+    const int h = f[i * S::LINES * S::LD * 2];
+    e = max(e, h & 0x7fffffff);
+    bits |= h ^ (h >> 31);
+  }
+  atomicMax(&k.word(S::I_F, dir), f64 ? e >> 20 : x + 4 - __clz(bits));
 }
 // The exponent the column's fluxes are read at: one bit of room.
 template <class O, int E>
 __device__ __forceinline__ int fx_line_exp(const FxBlock<O, E>& k, int dir) {
-  return (k.word(FxShape<O, E>::I_F, dir) >> 20) + 1;
+  return k.word(FxShape<O, E>::I_F, dir) + 1;
 }
 // The line projected along x_0, in the place of its values.
 template <class O, int E, int TAB>
-__device__ __forceinline__ void fx_line_project(const FxBlock<O, E>& k, int dir, int e) {
+__device__ __forceinline__ void fx_line_project(const FxBlock<O, E>& k, int dir, int e, bool f64, int x) {
   using S = FxShape<O, E>;
   constexpr int N = O::N;
-  double* f = k.f() + (dir * S::NS + k.line) * S::LD + k.col;
+  long long* t = k.m + S::O_F + (dir * S::NS + k.line) * S::LD + k.col;
   long long v[N];
+  if (f64) {
 #pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = fx_from_double(f[i * S::LINES * S::LD], e);
+    for (int i = 0; i < N; ++i) v[i] = fx_from_double(__longlong_as_double(t[i * S::LINES * S::LD]), e);
+  } else {
+    if (x >= e) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = t[i * S::LINES * S::LD] << (x - e);
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = fx_align(t[i * S::LINES * S::LD], e - x);
+    }
+  }
   const FxPairs<O> p(v);
-  long long* t = reinterpret_cast<long long*>(f);
 #pragma unroll
   for (int a = 0; a < N; ++a) t[a * S::LINES * S::LD] = p.template row<TAB>(a);
 }
@@ -277,41 +304,139 @@ __device__ __forceinline__ bool fx_task(int line, int j, int* dir, int* pre) {
   return i < O::D * O::FX_NPRE;
 }
 
-// Phases 2 to 5 of one slice: H from the spatial modes g (exponent and NaN
-// bits of the column given), fluxes, projections, accumulation.  kt < 0: the
-// first sweep's slice.  k: all columns, kf: those projected.
+// Phase 5: the last projection of the thread's tasks, v(b), and its products
+// with the slice's P_a(t) / N added to the accumulators (FIRST: the sums of
+// P_a0 / N, stored).
+template <class O, int E, bool FIRST>
+__device__ __forceinline__ void fx_accumulate(const FxBlock<O, E>& kf, int kt) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D, N = O::N, P = O::P, LD = S::LD;
+  FxCoef ct[N];
+#pragma unroll
+  for (int a = 0; a < N; ++a) ct[a] = FIRST ? O::fx_ssum(a) : O::fx_valt(a, kt);
+#pragma unroll 1
+  for (int j = 0; j < S::TASKS; ++j) {
+    int d, pre;
+    if (!fx_task<O, E>(kf.line, j, &d, &pre)) continue;
+    const FxPairs<O> p = fx_last<O, E>(kf, d, O::fx_pre_slot(pre));
+    const int deg = O::fx_pre_deg(pre), b0 = O::fx_pre_base(pre);
+    long long* acc = kf.m + S::O_A + d * O::NP_ST * LD + kf.col;
+    long long* q = acc + O::fx_first(b0) * LD;
+    if (!FIRST) {  // larger fluxes than in the slices before: what is there moves down
+      const int up = kf.word(S::I_UP, d);
+      if (up > 0) {
+        const int cnt = (P - deg + 1) * (P - deg + 2) / 2;
+#pragma unroll 1
+        for (int i = 0; i < cnt; ++i) q[i * LD] = fx_align(q[i * LD], up);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      if (n > P - deg) break;
+      const long long v = p.template row<FX_P>(n);
+      const int h = fx_hi(v), l = fx_lo(v);
+#pragma unroll
+      for (int a = 0; a < N - n; ++a) {
+        if (a > P - deg - n) break;
+        FxSum s;
+        if (FIRST) {
+          s.mul(h, l, ct[a].h, ct[a].l);
+          acc[O::fx_init(b0 + n, a) * LD] = s.get();
+        } else {
+          s.add(q[a * LD]);
+          s.mul(h, l, ct[a].h, ct[a].l);
+          q[a * LD] = s.get();
+        }
+      }
+      q += (P - deg - n + 1) * LD;  // the next mode's
+    }
+  }
+}
+
+// Phases 2 to 5 of one slice: H from the spatial modes g, fluxes, projections,
+// accumulation.  kt < 0: the first sweep's slice (g = U).  k: all columns, kf:
+// those projected.
 template <class O, int E>
 __device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxBlock<O, E>& kf, const long long* g,
-                                               int eg, int nan_bits, const FxCoef* c1, const FxCoef* c2, int kt,
-                                               double gm1) {
+                                               const FxCoef* c1, const FxCoef* c2, int kt, double gm1,
+                                               const FxFactor& gm1x) {
   using S = FxShape<O, E>;
   constexpr int D = O::D, Q = O::Q, N = O::N, P = O::P, LD = S::LD;
   if (k.act) {
     long long t[N];
     fx_line_modes<O, LD>(g + k.col, c1, c2, t);
-    double* h = k.f() + k.line * LD + k.col;
-    fx_line_points<O>(t, [&](int k0, long long v) { h[k0 * S::LINES * LD] = fx_to_double(v, eg, nan_bits); });
+    long long* h = k.m + S::O_F + k.line * LD + k.col;
+    int n = 0;
+    fx_line_points<O>(t, [&](int k0, long long v) {
+      h[k0 * S::LINES * LD] = v;
+      n = max(n, __clz((int)(v >> 32)));
+    });
+    if (k.col % Q == 0) atomicMax(&k.word(S::I_N), n);
   }
   fx_sync<S::NT>();
+  // fluxes; an element with a point that is not for the integers (or with
+  // exponents near the range of doubles) has all of its points in FP64
+  const int* wx = k.w + (kt < 0 ? S::I_EU : S::I_EH);
+  long long u[S::PTS][Q];
+  bool bad = false;
 #pragma unroll
   for (int r = 0; r < S::PTS; ++r) {
     const int it = threadIdx.x + r * S::NT;
     if (it < E * S::NS) {
-      double* base = k.f() + (it % S::NS) * LD + (it / S::NS) * Q;
-      double u[Q], F[D * Q];
+      const int c0 = (it / S::NS) * Q, m = it % S::NS;
+      long long* base = k.m + S::O_F + m * LD + c0;
 #pragma unroll
-      for (int v = 0; v < Q; ++v) u[v] = base[v];
-      euler_flux_all<D, double>(u, gm1, F);
+      for (int v = 0; v < Q; ++v) u[r][v] = base[v];
+      int em[D], range = max(abs(wx[c0] - 1022), abs(wx[c0 + D + 1] - 1022));
 #pragma unroll
-      for (int d = 0; d < D; ++d)
+      for (int d = 0; d < D; ++d) {
+        em[d] = wx[c0 + d + 1];
+        range = max(range, em[d] - 1022);
+      }
+      const int n = k.w[S::I_N + c0];
+      const FxFluxExp<D> x(em, wx[c0 + D + 1], wx[c0], n, gm1x.ef);
+      long long F[D][D + 1];
+      if (range < 480 && fx_euler_flux<D>(u[r], x, wx[c0 + D + 1], n, gm1x, F)) {
 #pragma unroll
-        for (int v = 1; v < Q; ++v) base[d * S::NS * LD + v] = F[d * Q + v];
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+          for (int v = 1; v < Q; ++v) base[d * S::NS * LD + v] = F[d][v - 1];
+      } else {
+        k.w[S::I_F64 + c0] = 1;
+        bad = true;
+      }
+      if (m == 0) {
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+          for (int v = 1; v < Q; ++v) k.w[S::I_X + d * S::C + c0 + v] = x.flux(d, v, em);
+      }
     }
   }
-  fx_sync<S::NT>();
+  if (__syncthreads_or(bad)) {
+#pragma unroll
+    for (int r = 0; r < S::PTS; ++r) {
+      const int it = threadIdx.x + r * S::NT;
+      if (it < E * S::NS && k.w[S::I_F64 + (it / S::NS) * Q]) {
+        const int c0 = (it / S::NS) * Q;
+        double* base = k.f() + (it % S::NS) * LD + c0;
+        double ud[Q], F[D * Q];
+#pragma unroll
+        for (int v = 0; v < Q; ++v)
+          ud[v] = fx_to_double(u[r][v], wx[c0 + v], kt < 0 ? fx_poison(wx[c0 + v]) : k.w[S::I_NAN + c0 + v]);
+        euler_flux_all<D, double>(ud, gm1, F);
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+          for (int v = 1; v < Q; ++v) base[d * S::NS * LD + v] = F[d * Q + v];
+      }
+    }
+    fx_sync<S::NT>();
+  }
+  const bool f64 = kf.act && k.w[S::I_F64 + kf.col / Q * Q];
   if (kf.act) {
 #pragma unroll 1
-    for (int d = 0; d < D; ++d) fx_line_max<O, E>(kf, d);
+    for (int d = 0; d < D; ++d) fx_line_max<O, E>(kf, d, f64, kf.word(S::I_X, d));
   }
   fx_sync<S::NT>();
   if (kf.act) {
@@ -322,10 +447,11 @@ __device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxB
         kf.word(S::I_UP, d) = kt > 0 ? e - kf.word(S::I_EA, d) : 0;
         kf.word(S::I_EA, d) = e;
       }
-      fx_line_project<O, E, FX_P>(kf, d, e);
+      fx_line_project<O, E, FX_P>(kf, d, e, f64, kf.word(S::I_X, d));
     }
   }
   fx_sync<S::NT>();
+  if (k.act && k.line == 0 && k.col % Q == 0) k.word(S::I_N) = k.word(S::I_F64) = 0;
   if constexpr (D == 3) {
     if (kf.act) {
 #pragma unroll 1
@@ -334,38 +460,10 @@ __device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxB
     fx_sync<S::NT>();
   }
   if (!kf.act) return;
-  FxCoef ct[N];
-#pragma unroll
-  for (int a = 0; a < N; ++a) ct[a] = kt < 0 ? O::fx_ssum(a) : O::fx_valt(a, kt);
-#pragma unroll 1
-  for (int j = 0; j < S::TASKS; ++j) {
-    int d, pre;
-    if (!fx_task<O, E>(kf.line, j, &d, &pre)) continue;
-    const FxPairs<O> p = fx_last<O, E>(kf, d, O::fx_pre_slot(pre));
-    const int deg = O::fx_pre_deg(pre), b0 = O::fx_pre_base(pre);
-    const int up = kf.word(S::I_UP, d);
-    long long* acc = kf.m + S::O_A + d * O::NP_ST * LD + kf.col;
-    long long* q = acc + O::fx_first(b0) * LD;
-#pragma unroll
-    for (int n = 0; n < N; ++n) {
-      if (n > P - deg) break;
-      const long long v = p.template row<FX_P>(n);
-      const int h = fx_hi(v), l = fx_lo(v);
-#pragma unroll
-      for (int a = 0; a < N - n; ++a) {
-        if (a > P - deg - n) break;
-        FxSum s;
-        s.mul(h, l, ct[a].h, ct[a].l);
-        if (kt < 0) {
-          acc[O::fx_init(b0 + n, a) * LD] = s.get();
-        } else {
-          if (kt > 0) s.add(up > 0 ? fx_align(q[a * LD], up) : q[a * LD]);
-          q[a * LD] = s.get();
-        }
-      }
-      q += (P - deg - n + 1) * LD;  // the next mode's
-    }
-  }
+  if (kt < 0)
+    fx_accumulate<O, E, true>(kf, kt);
+  else
+    fx_accumulate<O, E, false>(kf, kt);
 }
 
 // z_d = Dt/dx_d C_d acc_d of the thread's rows; of the mass column K_d times
@@ -389,9 +487,11 @@ __device__ __forceinline__ void fx_changes(const FxBlock<O, E>& k, const FxFacto
       z[r][d] = 0;
       if (n < O::NP_ST) {
         const int j1 = O::fx_row(table, n + 1);
+        int j = O::fx_row(table, n), i = 0;
+        if (j == j1) continue;
         FxSum s;
 #pragma unroll 1
-        for (int j = O::fx_row(table, n), i = 0; j < j1; ++j) {
+        for (; j < j1; ++j) {
           const int c = O::fx_col(j);
           if (c >= nv) break;
           s.mul(v[c * S::LD], O::fx_cval(j));
@@ -459,13 +559,20 @@ __device__ __forceinline__ void fx_update(const FxBlock<O, E>& k, const FxFactor
 #pragma unroll
     for (int r = 0; r < S::ROWS; ++r) {
       const int n = k.line + r * S::LINES;
-      if (n < O::NP_ST) k.m[S::O_H + n * S::LD + k.col] = fx_move(z[r][0], -up);
+      if (n < O::NP_ST) {
+        k.m[S::O_H + n * S::LD + k.col] = fx_move(z[r][0], -up);
+#pragma unroll
+        for (int d = 0; d < D; ++d) k.m[S::O_A + (d * O::NP_ST + n) * S::LD + k.col] = 0;
+      }
     }
     if (k.line == 0) {
       k.word(S::I_EH) = top - up;
       k.word(S::I_NAN) = nan_bits | fx_poison(top - up);
 #pragma unroll
-      for (int d = 0; d < D; ++d) k.word(S::I_Z, d) = k.word(S::I_F, d) = 0;
+      for (int d = 0; d < D; ++d) {
+        k.word(S::I_Z, d) = 0;
+        k.word(S::I_F, d) = kFxNoExp;
+      }
     }
   }
   fx_sync<S::NT>();
@@ -583,13 +690,13 @@ __device__ __forceinline__ void fx_volume_term(const FxBlock<O, E>& k) {
   constexpr int D = O::D;
   if (k.act) {
 #pragma unroll 1
-    for (int d = 0; d < D; ++d) fx_line_max<O, E>(k, d);
+    for (int d = 0; d < D; ++d) fx_line_max<O, E>(k, d, true, 0);
   }
   fx_sync<S::NT>();
   if (k.act) {
-    fx_line_project<O, E, FX_D>(k, 0, fx_line_exp<O, E>(k, 0));
+    fx_line_project<O, E, FX_D>(k, 0, fx_line_exp<O, E>(k, 0), true, 0);
 #pragma unroll 1
-    for (int d = 1; d < D; ++d) fx_line_project<O, E, FX_W>(k, d, fx_line_exp<O, E>(k, d));
+    for (int d = 1; d < D; ++d) fx_line_project<O, E, FX_W>(k, d, fx_line_exp<O, E>(k, d), true, 0);
   }
   fx_sync<S::NT>();
   if constexpr (D == 3) {
@@ -647,6 +754,7 @@ __device__ __forceinline__ void fx_predictor_chunk(const PredictorArgs& a, char*
     cf[d] = fx_factor(c[d]);
   }
   const double gm1 = a.gamma - 1.0;
+  const FxFactor gm1x = fx_factor(gm1);
   const FxModes<O, E> md(k);
   FxCoef c1[N], c2[N];
   fx_load_coefs<O>(D == 2 ? k.line % N : (k.line / N) % N, c1);
@@ -660,9 +768,12 @@ __device__ __forceinline__ void fx_predictor_chunk(const PredictorArgs& a, char*
   if (k.act && k.line == 0) {
     const int eu = fx_norm_exp<NP_S>(ud + k.col, LD);
     k.word(S::I_EU) = eu;
-    k.word(S::I_SUM) = 0;
+    k.word(S::I_SUM) = k.word(S::I_N) = k.word(S::I_F64) = 0;
 #pragma unroll
-    for (int d = 0; d < D; ++d) k.word(S::I_Z, d) = k.word(S::I_F, d) = 0;
+    for (int d = 0; d < D; ++d) {
+      k.word(S::I_Z, d) = 0;
+      k.word(S::I_F, d) = kFxNoExp;
+    }
     if (a.ubar_old && live) a.ubar_old[(size_t)e * Q + q] = ud[k.col];
   }
   fx_sync<S::NT>();
@@ -673,19 +784,17 @@ __device__ __forceinline__ void fx_predictor_chunk(const PredictorArgs& a, char*
 
   // the first sweep on U, then the others (AmrDG.h:1103-1119)
   {
-    const int eu = k.act ? k.word(S::I_EU) : 0;
-    fx_sweep_slice<O, E>(k, kf, k.m + S::O_U, eu, fx_poison(eu), c1, c2, -1, gm1);
+    fx_sweep_slice<O, E>(k, kf, k.m + S::O_U, c1, c2, -1, gm1, gm1x);
     fx_sync<S::NT>();
     fx_update<O, E>(k, cf, true);
   }
 #pragma unroll 1
   for (int s = 1; s < a.sweeps; ++s) {
     if (k.act && k.line == 0) k.word(S::I_SUM) = 0;
-    const int eh = k.act ? k.word(S::I_EH) : 0, nan_bits = k.act ? k.word(S::I_NAN) : 0;
 #pragma unroll 1
     for (int kt = 0; kt < N; ++kt) {
       fx_time_slice<O, E>(k, md, kt);
-      fx_sweep_slice<O, E>(k, kf, k.m + S::O_G, eh, nan_bits, c1, c2, kt, gm1);
+      fx_sweep_slice<O, E>(k, kf, k.m + S::O_G, c1, c2, kt, gm1, gm1x);
     }
     fx_sync<S::NT>();
     fx_update<O, E>(k, cf, false);

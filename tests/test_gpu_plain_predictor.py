@@ -43,6 +43,30 @@ def test_step_matches_oracle(D, P, n, ic, E):
     assert np.max(np.abs(a - b)) < 1e-13 * np.max(np.abs(b[:, :, 0]))
 
 
+@pytest.mark.parametrize("D,P", [(2, 1), (2, 3), (2, 4), (3, 1), (3, 2)])
+@pytest.mark.parametrize("slope", [0.5, 0.98])
+def test_steep_densities_and_low_pressures_match_oracle(D, P, slope):
+    """Densities up to 100 apart within an element, and pressures down to the
+    floor beside ordinary ones: both flux evaluations and their border."""
+    o, g = pair(D, P, (6, 5, 1) if D == 2 else (4, 3, 3), "vortex" if D == 2 else "blast3d")
+    r = np.random.RandomState(P)
+    U = np.zeros_like(o.get_uw())
+    n = len(U)
+    lin = 1  # the first mode of degree one
+    U[:, 0, 0] = r.uniform(1, 2, n)
+    U[::2, 0, lin] = slope * U[::2, 0, 0]
+    U[:, 1:D + 1, 0] = 0.02 * r.uniform(-1, 1, (n, D))
+    U[:, D + 1, 0] = np.where(np.arange(n) % 3 == 0, 1e-14, 1.0)
+    o.set_uw(U, 0)
+    g.set_U_w(U)
+    o.dt = g.Dt = 1e-4
+    o.ader()
+    g.ADER()
+    a, b = g.get_U_w(), o.get_uw()
+    assert np.isfinite(b).all()
+    assert np.max(np.abs(a - b)) < 1e-13 * np.max(np.abs(b[:, :, 0]))
+
+
 @pytest.mark.parametrize("D,P", [(2, 1), (2, 2), (2, 3), (2, 6), (3, 2), (3, 3)])
 def test_step_scales_with_the_state(D, P):
     """The Euler fluxes are homogeneous of degree one where the pressure is above
