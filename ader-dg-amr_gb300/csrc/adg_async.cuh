@@ -1,6 +1,6 @@
-// Asynchronous copies on sm_103a: mbarrier phases with bounded waits and
-// 1D bulk copies (cp.async.bulk, the TMA engine's untiled form) from global
-// into shared memory.  A bulk copy needs 16-byte aligned addresses and a size
+// Asynchronous copies on sm_103a: mbarrier phases with bounded waits, 8-byte
+// copies of a thread's own, and 1D bulk copies (cp.async.bulk, the TMA
+// engine's untiled form) from global into shared memory.  A bulk copy needs 16-byte aligned addresses and a size
 // that is a multiple of 16 bytes.
 #pragma once
 
@@ -40,6 +40,11 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// Eight bytes per thread from global into shared memory, without a register.
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 }  // namespace tc
 }  // namespace adg

@@ -544,7 +544,8 @@ int launch_ghost_fill(adg_ctx* ctx) {
   const Hierarchy& H = ctx->hier;
   if (!H.gf_elem.empty()) {
     ScatterArgs sa{};
-    sa.Uw = ctx->Uw.p;
+    sa.fine = ctx->Uw.p;
+    sa.coarse = ctx->Uw.p;
     sa.dst = ctx->gf_elem.p;
     sa.parent = ctx->gf_parent.p;
     sa.child = ctx->gf_child.p;
@@ -965,8 +966,9 @@ int apply_layout(adg_ctx* ctx, const std::vector<std::vector<amr::IBox>>& ng,
     const size_t o = lo[l], n = lo[l + 1] - lo[l];
     if (!n) continue;
     ScatterArgs sa{};
-    sa.Uw = nU;
-    sa.Uw_old = ctx->Uw.p;
+    sa.fine = nU;
+    sa.coarse = nU;
+    sa.old = ctx->Uw.p;
     sa.dst = ctx->remap_i.p + o;
     sa.parent = ctx->remap_i.p + nr + o;
     sa.src_old = ctx->remap_i.p + 2 * nr + o;
@@ -1376,7 +1378,8 @@ int adg_init(adg_ctx* ctx) {
     ADG_CUDA(cudaMemcpyAsync(d_par.p, par.data(), dst.size() * 4, cudaMemcpyHostToDevice, ctx->stream), "h2d");
     ADG_CUDA(cudaMemcpyAsync(d_ch.p, ch.data(), dst.size(), cudaMemcpyHostToDevice, ctx->stream), "h2d");
     ScatterArgs sa{};
-    sa.Uw = ctx->Uw.p;
+    sa.fine = ctx->Uw.p;
+    sa.coarse = ctx->Uw.p;
     sa.dst = d_dst.p;
     sa.parent = d_par.p;
     sa.child = d_ch.p;

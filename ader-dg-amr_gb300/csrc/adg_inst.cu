@@ -192,28 +192,30 @@ struct Impl final : KernelSet {
     return cudaGetLastError();
   }
   cudaError_t average_down(double* Uw, const int* rec, int nrec, cudaStream_t s) const override {
-    if (nrec <= 0) return cudaSuccess;
-    constexpr int RB = ad_records_per_block<O>();
-    k_average_down<O><<<(unsigned)((nrec + RB - 1) / RB), dim3(RB * O::Q, 1 << O::D), 0, s>>>(Uw, rec, nrec);
-    return cudaGetLastError();
+    return gather(Uw, Uw, rec, nrec, s);
   }
   cudaError_t scatter(const ScatterArgs& a, cudaStream_t s) const override {
-    const long long n = (long long)a.n * O::Q;
-    if (n == 0) return cudaSuccess;
-    k_scatter<O><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a);
+    if (a.n <= 0) return cudaSuccess;
+    constexpr int NT = TransferShape<O>::NT_S;
+    k_scatter<O><<<(unsigned)((a.n * O::Q + NT - 1) / NT), NT, 0, s>>>(a);
     return cudaGetLastError();
   }
   cudaError_t interp_scatter(const double* coarse, const int8_t* child, long long n, double* fine,
                              cudaStream_t s) const override {
-    if (n <= 0) return cudaSuccess;
-    const long long t = n * O::Q;
-    k_interp_scatter<O><<<(unsigned)((t + 127) / 128), 128, 0, s>>>(coarse, child, n, fine);
-    return cudaGetLastError();
+    ScatterArgs a{};
+    a.fine = fine;
+    a.coarse = coarse;
+    a.child = child;
+    a.n = n;
+    return scatter(a, s);
   }
   cudaError_t interp_gather(const double* fine, long long n, double* coarse, cudaStream_t s) const override {
+    return gather(fine, coarse, nullptr, n, s);
+  }
+  static cudaError_t gather(const double* fine, double* coarse, const int* rec, long long n, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    const long long t = n * O::Q;
-    k_interp_gather<O><<<(unsigned)((t + 127) / 128), 128, 0, s>>>(fine, n, coarse);
+    constexpr int B = TransferShape<O>::GATHER;
+    k_gather<O><<<(unsigned)((n + B - 1) / B), TransferShape<O>::NT_G, 0, s>>>(fine, coarse, rec, n);
     return cudaGetLastError();
   }
   cudaError_t tag(const TagArgs& a, cudaStream_t s) const override {

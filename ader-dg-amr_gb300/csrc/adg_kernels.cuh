@@ -956,25 +956,6 @@ __global__ void k_numflux_split(FaceArgs a) {
 
 // Runtime child / face index dispatch to the compile-time generated
 // coarse-fine operators.
-template <class O, class In, class Out>
-__device__ __forceinline__ void pcf_rt(int l, const In& in, Out out) {
-  switch (l) {
-    case 0: O::template pcf<0>(in, out); break;
-    case 1: O::template pcf<1>(in, out); break;
-    case 2: O::template pcf<2>(in, out); break;
-    case 3: O::template pcf<3>(in, out); break;
-    default:
-      if constexpr (O::D == 3) {
-        switch (l) {
-          case 4: O::template pcf<4>(in, out); break;
-          case 5: O::template pcf<5>(in, out); break;
-          case 6: O::template pcf<6>(in, out); break;
-          default: O::template pcf<7>(in, out); break;
-        }
-      }
-  }
-}
-
 template <class O, int DD, int S, class In, class Out>
 __device__ __forceinline__ void pflux_mom_k(int k, const In& in, Out out) {
   if constexpr (O::D == 2) {
@@ -1507,177 +1488,6 @@ __global__ void k_init_ic(ICArgs a) {
   }
 }
 
-
-// ===========================================================================
-// AMR transfer kernels (L2ProjInterp, Source/NumericalMethod/AmrDG/AmrDG_Interpolater.tpp)
-// One thread per (element, variable) column; runtime child / face indices are
-// dispatched to the compile-time generated operators.
-// ===========================================================================
-// average_down / amr_gather (AmrDG_Interpolater.tpp:283-342, 366-398):
-// u_c = 2^-D Minv sum_l P_fc[l] u_f[l].  rec: coarse, fine_0 .. fine_{2^D-1}.
-// Block (32, 2^D): warp l projects child l of 32 (record, variable) pairs, so
-// every warp runs one operator; warp 0 sums the children in order.
-// Records per block of k_average_down.
-template <class O>
-constexpr int ad_records_per_block() {
-  return O::D == 2 ? 8 : 4;
-}
-
-// Block (RB Q, 2^D): records r0 .. r0+RB-1; the children's states are staged
-// in shared memory with coalesced 16-byte loads (each element's Q Np_s
-// doubles are contiguous), thread (r, q, child) projects one child, row 0
-// sums and scales, and the coarse states leave through shared memory again.
-template <class O>
-__global__ void k_average_down(double* Uw, const int* rec, int nrec) {
-  constexpr int D = O::D, Q = O::Q, NP_S = O::NP_S, NOV = 1 << D, RB = ad_records_per_block<O>();
-  constexpr int EL = Q * NP_S, EL2 = EL / 2, NT = RB * Q * NOV;
-  static_assert(EL % 2 == 0, "element blocks must be whole 16-byte units");
-  __shared__ __align__(16) double fine[NOV * RB * EL];
-  __shared__ double part[NOV][NP_S][RB * Q + 1];
-  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-  const int r0 = blockIdx.x * RB;
-  const int nr = nrec - r0 < RB ? nrec - r0 : RB;
-  for (int i = tid; i < NOV * nr * EL2; i += NT) {
-    const int L = i / (nr * EL2), rem = i % (nr * EL2);
-    const int r = rem / EL2, off = rem % EL2;
-    const int e = rec[(size_t)(r0 + r) * (NOV + 1) + 1 + L];
-    reinterpret_cast<double2*>(fine)[(L * RB + r) * EL2 + off] =
-        __ldg(reinterpret_cast<const double2*>(Uw + (size_t)e * EL) + off);
-  }
-  __syncthreads();
-  const int x = threadIdx.x, L = threadIdx.y;
-  const int r = x / Q, q = x % Q;
-  if (r < nr) {
-    const double* uf = fine + (L * RB + r) * EL + q * NP_S;
-    double tmp[NP_S];
-    switch (L) {
-      case 0: O::template pfc<0>(RegIn{uf}, RegOut{tmp}); break;
-      case 1: O::template pfc<1>(RegIn{uf}, RegOut{tmp}); break;
-      case 2: O::template pfc<2>(RegIn{uf}, RegOut{tmp}); break;
-      case 3: O::template pfc<3>(RegIn{uf}, RegOut{tmp}); break;
-      default:
-        if constexpr (D == 3) {
-          switch (L) {
-            case 4: O::template pfc<4>(RegIn{uf}, RegOut{tmp}); break;
-            case 5: O::template pfc<5>(RegIn{uf}, RegOut{tmp}); break;
-            case 6: O::template pfc<6>(RegIn{uf}, RegOut{tmp}); break;
-            default: O::template pfc<7>(RegIn{uf}, RegOut{tmp}); break;
-          }
-        }
-    }
-#pragma unroll
-    for (int n = 0; n < NP_S; ++n) part[L][n][x] = tmp[n];
-  }
-  __syncthreads();
-  double* out = fine;  // the children are consumed: [RB][EL] coarse states
-  // mode n of every (record, variable) summed by row n mod 2^D: the FP64 work
-  // of the sums spread over all warps (and so over the SM's four schedulers)
-  if (r < nr) {
-#pragma unroll
-    for (int n0 = 0; n0 < NP_S; n0 += NOV) {
-      const int n = n0 + L;
-      if (n < NP_S) {
-        double sum = 0.0;
-#pragma unroll
-        for (int l = 0; l < NOV; ++l) sum = __dadd_rn(sum, part[l][n][x]);  // as k_interp_gather
-        out[r * EL + q * NP_S + n] = (1.0 / NOV) * (O::minv(n) * sum);
-      }
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < nr * EL2; i += NT) {
-    const int rr = i / EL2, off = i % EL2;
-    reinterpret_cast<double2*>(Uw + (size_t)rec[(size_t)(r0 + rr) * (NOV + 1)] * EL)[off] =
-        reinterpret_cast<const double2*>(out)[rr * EL2 + off];
-  }
-}
-
-// L2ProjInterp on caller batches (AmrDG_Interpolater.tpp:344-398): thread
-// per (cell, variable).  Scatter: fine[i] = Minv P_cf[child[i]] coarse[i];
-// gather: coarse[i] = 2^-D Minv sum_l P_fc[l] fine[i][l], children summed in
-// order as k_average_down does.  Layouts [n][Q][Np_s] and [n][2^D][Q][Np_s].
-template <class O>
-__global__ void k_interp_scatter(const double* coarse, const int8_t* child, long long n, double* fine) {
-  constexpr int Q = O::Q, NP_S = O::NP_S;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * Q) return;
-  const long long i = t / Q;  // cell; variable t % Q
-  double out[NP_S];
-  const int l = child[i];
-#pragma unroll
-  for (int k = 0; k < NP_S; ++k) out[k] = __longlong_as_double(0x7ff8000000000000LL);  // NaN: child out of range
-  if (l >= 0 && l < (1 << O::D)) pcf_rt<O>(l, RegIn{coarse + (size_t)t * NP_S}, RegOut{out});
-#pragma unroll
-  for (int k = 0; k < NP_S; ++k) fine[(size_t)t * NP_S + k] = out[k];
-}
-
-template <class O>
-__global__ void k_interp_gather(const double* fine, long long n, double* coarse) {
-  constexpr int D = O::D, Q = O::Q, NP_S = O::NP_S, NOV = 1 << D;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n * Q) return;
-  const long long i = t / Q;
-  const int q = (int)(t % Q);
-  double part[NOV][NP_S];
-#pragma unroll
-  for (int l = 0; l < NOV; ++l) {
-    const double* uf = fine + (((size_t)i * NOV + l) * Q + q) * NP_S;
-    switch (l) {
-      case 0: O::template pfc<0>(RegIn{uf}, RegOut{part[l]}); break;
-      case 1: O::template pfc<1>(RegIn{uf}, RegOut{part[l]}); break;
-      case 2: O::template pfc<2>(RegIn{uf}, RegOut{part[l]}); break;
-      case 3: O::template pfc<3>(RegIn{uf}, RegOut{part[l]}); break;
-      default:
-        if constexpr (D == 3) {
-          switch (l) {
-            case 4: O::template pfc<4>(RegIn{uf}, RegOut{part[l]}); break;
-            case 5: O::template pfc<5>(RegIn{uf}, RegOut{part[l]}); break;
-            case 6: O::template pfc<6>(RegIn{uf}, RegOut{part[l]}); break;
-            default: O::template pfc<7>(RegIn{uf}, RegOut{part[l]}); break;
-          }
-        }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < NP_S; ++k) {
-    double sum = 0.0;
-#pragma unroll
-    for (int l = 0; l < NOV; ++l) sum = __dadd_rn(sum, part[l][k]);  // never fused with a child's last product
-    coarse[(size_t)t * NP_S + k] = (1.0 / NOV) * (O::minv(k) * sum);
-  }
-}
-
-// Coarse -> fine projection (amr_scatter, AmrDG_Interpolater.tpp:344-364)
-// into ghost elements (FillPatchTwoLevels) or, with src_old, the regrid
-// remap of a level (valid data of the old layout where it existed).
-struct ScatterArgs {
-  double* Uw;            // destination array (and coarse source)
-  const double* Uw_old;  // optional: old layout's state
-  const int* dst;        // [n] destination element
-  const int* parent;     // [n] coarse parent element in Uw
-  const int8_t* child;   // [n] child index
-  const int* src_old;    // optional [n]: element in Uw_old, -1 = project
-  int n;
-};
-
-template <class O>
-__global__ void k_scatter(ScatterArgs a) {
-  constexpr int Q = O::Q, NP_S = O::NP_S;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)a.n * Q) return;
-  const int i = (int)(t / Q), q = (int)(t % Q);
-  double* dst = a.Uw + ((size_t)a.dst[i] * Q + q) * NP_S;
-  if (a.src_old && a.src_old[i] >= 0) {
-    const double* s = a.Uw_old + ((size_t)a.src_old[i] * Q + q) * NP_S;
-#pragma unroll
-    for (int n = 0; n < NP_S; ++n) dst[n] = s[n];
-    return;
-  }
-  double v[NP_S];
-  pcf_rt<O>(a.child[i], RegIn{a.Uw + ((size_t)a.parent[i] * Q + q) * NP_S}, RegOut{v});
-#pragma unroll
-  for (int n = 0; n < NP_S; ++n) dst[n] = v[n];
-}
 
 // Refinement indicator on cell means (mode 0), tag when above threshold:
 // kind 0 normalised density gradient max_d |rho(i+e_d)-rho(i-e_d)|/(2 rho(i)),

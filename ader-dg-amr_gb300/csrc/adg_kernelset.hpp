@@ -8,6 +8,7 @@
 
 #include "adg_kernels.cuh"
 #include "adg_seed_tc.cuh"
+#include "adg_transfer.cuh"
 
 namespace adg {
 

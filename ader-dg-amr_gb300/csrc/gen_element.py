@@ -873,6 +873,23 @@ def emit_fx(el, ops):
         kshifts.append(math.ceil(math.log2(max(abs(v) for r in KS[d] for _, v in r)) - 1e-9))
         sparse.append((rows, shifts[d]))
     sparse += [(KS[d], kshifts[d]) for d in range(D)]
+    # projections between levels along one dimension, exact dyadic fractions:
+    # P_n((x + 1) / 2) in the P_j, and the transposed projection's coefficients
+    # (Minv included), one word over 2^FX_XG_GROW, the bound of their sums
+    c = legendre_shift_coeffs(P, True)
+    g = [[c[n][j] * Fraction(2 * n + 1, 2 * j + 1) for j in range(N)] for n in range(N)]
+    grow = 1 if max(sum(map(abs, r)) for r in g) <= 2 else 2
+    assert max(sum(map(abs, r)) for r in g) <= 1 << grow
+    mem.append(f"  static constexpr int FX_XG_GROW = {grow};")
+    word = [x * 2 ** (FX_LIMB - grow) for r in g for x in r]
+    assert all(x.denominator == 1 and abs(x) <= 1 << FX_LIMB for x in word)
+    half = [x * 64 for r in c for x in r]
+    assert all(x.denominator == 1 for x in half)
+    for fn, typ, v in (("fx_xg", "int", [int(x) for x in word]), ("xs", "double", [f"{int(x)} / 64.0" for x in half])):
+        mem.append(f"  static constexpr __host__ __device__ {typ} {fn}(int n, int j) {{ const int i = n * {N} + j; "
+                   f"return {select(v)}; }}")
+    modes = [el.mi_s.index(m) if sum(m) <= P else 0 for m in itertools.product(range(N), repeat=D)]
+    mem.append(f"  static constexpr __host__ __device__ int fx_mode(int i) {{ return {select(modes)}; }}")
     # (short rows are summed without folding the middle products in between)
     assert el.Np_st > 20 or max(len(r) for rr, _ in sparse for r in rr) <= 5
     # one table of rows: C_0 .. C_{D-1}, K_0 .. K_{D-1}
@@ -935,7 +952,6 @@ def add_ic_proj(el, ops):
 def add_amr_ops(el, ops):
     """L2ProjInterp operators (AmrDG_Interpolater.tpp:85-231), each an exact
     sum of products of the double-valued tables, rounded once:
-      pcf{l}      = Minv P_cf[l]              coarse -> fine child l (amr_scatter)
       pfc{l}      = P_fc[l]                   fine child l -> coarse (amr_gather)
       pflux{d}{s}{k} = P_flux_fc_{low,high}[d][k]  fine face points -> coarse face modes
     Child l of P_cf / P_fc: bit (D-1-d) of l is the upper half in direction d.
@@ -962,14 +978,9 @@ def add_amr_ops(el, ops):
                 v *= Fraction(tbl[n[d]][pt[d]])
             return v
 
-        Pcf = [[sum(quad[j][qi] * phi_child(ms[m], pt) for qi, pt in enumerate(el.pts_s)) for m in range(len(ms))]
-               for j in range(len(ms))]
         Pfc = [[sum(quad[m][qi] * phi_child(ms[j], pt) for qi, pt in enumerate(el.pts_s)) for m in range(len(ms))]
                for j in range(len(ms))]
-        cf = [[float(minv[j] * Pcf[j][m]) for m in range(len(ms))] for j in range(len(ms))]
         fc = [[float(Pfc[j][m]) for m in range(len(ms))] for j in range(len(ms))]
-        ops[f"pcf{l}"] = ([Stage(len(ms), len(ms), [[(c, r[c]) for c in range(len(ms)) if r[c] != 0.0] for r in cf])],
-                          len(ms), len(ms))
         ops[f"pfc{l}"] = ([Stage(len(ms), len(ms), [[(c, r[c]) for c in range(len(ms)) if r[c] != 0.0] for r in fc])],
                           len(ms), len(ms))
     nfc = 1 << (D - 1)
@@ -1272,7 +1283,6 @@ def generate(D, P, out_path):
     hdr.append(f"  static constexpr __host__ __device__ float time_val_f(int a, int k) {{ return "
                + select(f"(a * {N} + k)", tv, lambda v: lit(v) + "f") + "; }")
     hdr.append(disp("bd_term", [((d, s), f"bd_term{d}{s}") for d in range(D) for s in range(2)], ["d", "s"]))
-    hdr.append(disp("pcf", [((l,), f"pcf{l}") for l in range(1 << D)], ["l"]))
     hdr.append(disp("pfc", [((l,), f"pfc{l}") for l in range(1 << D)], ["l"]))
     hdr.append(disp("pflux", [((d, s, k), f"pflux{d}{s}{k}") for d in range(D) for s in range(2)
                               for k in range(1 << (D - 1))], ["d", "s", "k"]))
