@@ -97,8 +97,8 @@ struct adg_seed {
   bool normalised = false;
   DevBuf<float> X, T;  // data set
   long long nsamp = 0;
-  DevBuf<float> Z1, A1, Z2, A2, Z3, A3, Y, dY, dA, dZ, Xb, Tb;
-  DevBuf<float> red;  // partial sums of the split reductions (added in a fixed order)
+  DevBuf<float> Z1, A1, Z2, A2, Z3, A3, dY, dA, dZ, Xb, Tb;
+  DevBuf<float> red;  // slices of the weight gradients (added in order)
   long long work_rows = 0;
   DevBuf<int> idx;
   DevBuf<double> loss;
@@ -111,7 +111,7 @@ struct adg_seed {
   bool packed = false;
   ~adg_seed() {
     DevBuf<float>* bufs[] = {&params, &grads, &am, &av, &x_mean, &x_istd, &y_mean, &y_std, &X, &T,
-                             &Z1, &A1, &Z2, &A2, &Z3, &A3, &Y, &dY, &dA, &dZ, &Xb, &Tb, &wpack, &red};
+                             &Z1, &A1, &Z2, &A2, &Z3, &A3, &dY, &dA, &dZ, &Xb, &Tb, &wpack, &red};
     for (auto* b : bufs) b->release();
     idx.release();
     loss.release();
@@ -2463,27 +2463,42 @@ int adg_flops_per_element(int D, int P, double* algorithmic, double* issued) {
 // ===========================================================================
 namespace {
 
-// Few output tiles and a long K split K into slices whose partial sums go to
-// red (slice z at z M N) and are then added in slice order: the same result
-// on every run, unlike atomic accumulation.
-void sgemm(int TA, int TB, int M, int N, int K, const float* A, const float* B, float* C, const float* bias,
-           float* aux, int epi, cudaStream_t st, DevBuf<float>* red = nullptr) {
-  dim3 grid((N + 63) / 64, (M + 63) / 64, 1);
-  const int tiles = grid.x * grid.y;
-  const size_t mn = (size_t)M * N;
-  if (red && epi == mlp::EPI_STORE && tiles < 64 && K >= 512)
-    grid.z = (unsigned)std::min<size_t>(std::min(64, std::max(1, K / 256)), red->n / std::max<size_t>(mn, 1));
-  float* out = grid.z > 1 ? red->p : C;
-  if (!TA && !TB) mlp::k_sgemm<0, 0><<<grid, 256, 0, st>>>(M, N, K, A, B, out, bias, aux, epi);
-  else if (TA && !TB) mlp::k_sgemm<1, 0><<<grid, 256, 0, st>>>(M, N, K, A, B, out, bias, aux, epi);
-  else if (!TA && TB) mlp::k_sgemm<0, 1><<<grid, 256, 0, st>>>(M, N, K, A, B, out, bias, aux, epi);
-  else mlp::k_sgemm<1, 1><<<grid, 256, 0, st>>>(M, N, K, A, B, out, bias, aux, epi);
-  if (grid.z > 1) mlp::k_sum_slices<<<(unsigned)((mn + 255) / 256), 256, 0, st>>>((long long)mn, (int)grid.z, red->p, C);
+template <int TA, int TB, int EPI>
+void sgemm(const mlp::GemmArgs& g, cudaStream_t st) {
+  constexpr int T = mlp::kGemmTile;
+  const dim3 grid((g.N + T - 1) / T, (g.M + T - 1) / T, EPI == mlp::EPI_SLICE ? (g.K + g.kchunk - 1) / g.kchunk : 1);
+  mlp::k_sgemm<TA, TB, EPI><<<grid, mlp::kGemmThreads, 0, st>>>(g);
+}
+
+// Split of a weight gradient [M x N] over K samples: K range of a slice, so
+// that tiles times slices are about four blocks an SM (the 16384 samples'
+// gradients 15.8 us a layer; two blocks an SM 18.8), at least 64 samples each.
+int slice_chunk(int M, int N, int K) {
+  constexpr int T = mlp::kGemmTile;
+  const int tiles = ((M + T - 1) / T) * ((N + T - 1) / T);
+  const int ns = std::max(1, std::min(4 * 152 / tiles, K / 64));
+  return ((K + ns - 1) / ns + mlp::kGemmK - 1) / mlp::kGemmK * mlp::kGemmK;
+}
+
+// Slices of the gradients of a batch of B samples; total: floats of red.
+mlp::SliceTab slice_tab(const adg_seed* s, int B, size_t* total = nullptr) {
+  const int fin[4] = {s->n_in, s->h, s->h, s->h}, fout[4] = {s->h, s->h, s->h, s->n_out};
+  mlp::SliceTab t{};
+  long long base = 0;
+  for (int l = 0; l < 4; ++l) {
+    const int chunk = slice_chunk(fin[l], fout[l], B);
+    t.off[l] = (long long)s->off[2 * l];
+    t.base[l] = base;
+    t.ns[l] = (B + chunk - 1) / chunk;
+    base += (long long)t.ns[l] * (fin[l] + 1) * fout[l];
+    base = (base + 3) / 4 * 4;
+  }
+  t.off[4] = (long long)s->nparam;
+  if (total) *total = (size_t)base;
+  return t;
 }
 
 float* P(adg_seed* s, int k) { return s->params.p + s->off[k]; }
-float* G(adg_seed* s, int k) { return s->grads.p + s->off[k]; }
-
 cudaError_t seed_work(adg_seed* s, long long rows) {
   if (rows <= s->work_rows) return cudaSuccess;
   const size_t h = s->h;
@@ -2492,60 +2507,78 @@ cudaError_t seed_work(adg_seed* s, long long rows) {
     cudaError_t e = b->ensure((size_t)rows * h);
     if (e != cudaSuccess) return e;
   }
-  cudaError_t e = s->Y.ensure((size_t)rows * s->n_out);
-  if (e == cudaSuccess) {  // split-K slices of the weight gradients and the column-sum blocks
-    const size_t mn = std::max({(size_t)s->n_in * h, h * h, h * (size_t)s->n_out});
-    e = s->red.ensure(std::max(64 * mn, (size_t)128 * std::max(h, (size_t)s->n_out)));
-  }
-  if (e == cudaSuccess) e = s->dY.ensure((size_t)rows * s->n_out);
-  if (e == cudaSuccess) e = s->Xb.ensure((size_t)rows * s->n_in);
-  if (e == cudaSuccess) e = s->Tb.ensure((size_t)rows * s->n_out);
+  cudaError_t e = s->dY.ensure((size_t)rows * s->n_out);
   if (e == cudaSuccess) s->work_rows = rows;
   return e;
 }
 
-// Forward with stored pre-activations (training).
-void seed_forward_train(adg_seed* s, const float* X, int B, cudaStream_t st) {
-  using namespace mlp;
-  sgemm(0, 0, B, s->h, s->n_in, X, P(s, 0), s->A1.p, P(s, 1), s->Z1.p, EPI_BIAS_GELU, st);
-  sgemm(0, 0, B, s->h, s->h, s->A1.p, P(s, 2), s->A2.p, P(s, 3), s->Z2.p, EPI_BIAS_GELU, st);
-  sgemm(0, 0, B, s->h, s->h, s->A2.p, P(s, 4), s->A3.p, P(s, 5), s->Z3.p, EPI_BIAS_GELU, st);
-  sgemm(0, 0, B, s->n_out, s->h, s->A3.p, P(s, 6), s->Y.p, P(s, 7), nullptr, EPI_BIAS, st);
+mlp::GemmArgs gemm_args(int M, int N, int K, const float* A, const float* B, float* C) {
+  mlp::GemmArgs g{};
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  g.A = A;
+  g.B = B;
+  g.C = C;
+  return g;
 }
 
-// Backward from dY (in s->dY) into s->grads.
-// Column sums of X[M x N] by row blocks into red, then the blocks added in
-// order into out.
-void colsum(int M, int N, const float* X, float* out, DevBuf<float>& red, cudaStream_t st) {
-  dim3 grid((N + 127) / 128, std::max(1, std::min(128, M / 64)));
-  grid.y = (unsigned)std::max<size_t>(1, std::min<size_t>(grid.y, red.n / std::max(N, 1)));
-  mlp::k_colsum<<<grid, 128, 0, st>>>(M, N, X, red.p);
-  mlp::k_sum_slices<<<(unsigned)((N + 255) / 256), 256, 0, st>>>((long long)N, (int)grid.y, red.p, out);
+// Layer l of the forward pass on B rows; rows: sample rows of X.
+void forward_layer(adg_seed* s, int l, int B, const float* X, const int* rows, float* Z, float* A, cudaStream_t st) {
+  mlp::GemmArgs g = gemm_args(B, l < 3 ? s->h : s->n_out, l ? s->h : s->n_in, X, P(s, 2 * l), A);
+  g.bias = P(s, 2 * l + 1);
+  g.aux = Z;
+  g.rows = rows;
+  if (l < 3) sgemm<0, 0, mlp::EPI_BIAS_GELU>(g, st);
+  else sgemm<0, 0, mlp::EPI_BIAS>(g, st);
 }
 
-void seed_backward(adg_seed* s, const float* X, int B, cudaStream_t st) {
-  using namespace mlp;
+// Forward and backward pass of B samples: rows[i] (or i) of X and T.  The
+// pre-activations and dY stay on the device; the gradients' slices go to
+// s->red (layout: slice_tab), the sum of squared errors is added to s->loss.
+cudaError_t seed_pass(adg_seed* s, const float* X, const float* T, const int* rows, int B, cudaStream_t st) {
   const int h = s->h;
-  sgemm(1, 0, h, s->n_out, B, s->A3.p, s->dY.p, G(s, 6), nullptr, nullptr, EPI_STORE, st, &s->red);
-  colsum(B, s->n_out, s->dY.p, G(s, 7), s->red, st);
-  sgemm(0, 1, B, h, s->n_out, s->dY.p, P(s, 6), s->dZ.p, nullptr, s->Z3.p, EPI_GELU_BWD, st);  // dZ3
-  sgemm(1, 0, h, h, B, s->A2.p, s->dZ.p, G(s, 4), nullptr, nullptr, EPI_STORE, st, &s->red);
-  colsum(B, h, s->dZ.p, G(s, 5), s->red, st);
-  sgemm(0, 1, B, h, h, s->dZ.p, P(s, 4), s->dA.p, nullptr, s->Z2.p, EPI_GELU_BWD, st);  // dZ2
-  sgemm(1, 0, h, h, B, s->A1.p, s->dA.p, G(s, 2), nullptr, nullptr, EPI_STORE, st, &s->red);
-  colsum(B, h, s->dA.p, G(s, 3), s->red, st);
-  sgemm(0, 1, B, h, h, s->dA.p, P(s, 2), s->dZ.p, nullptr, s->Z1.p, EPI_GELU_BWD, st);  // dZ1
-  sgemm(1, 0, s->n_in, h, B, X, s->dZ.p, G(s, 0), nullptr, nullptr, EPI_STORE, st, &s->red);
-  colsum(B, h, s->dZ.p, G(s, 1), s->red, st);
+  size_t total = 0;
+  const mlp::SliceTab t = slice_tab(s, B, &total);
+  cudaError_t e = s->red.ensure(total);
+  if (e != cudaSuccess) return e;
+  forward_layer(s, 0, B, X, rows, s->Z1.p, s->A1.p, st);
+  forward_layer(s, 1, B, s->A1.p, nullptr, s->Z2.p, s->A2.p, st);
+  forward_layer(s, 2, B, s->A2.p, nullptr, s->Z3.p, s->A3.p, st);
+  mlp::GemmArgs y = gemm_args(B, s->n_out, h, s->A3.p, P(s, 6), s->dY.p);
+  y.bias = P(s, 7);
+  y.target = T;
+  y.target_rows = rows;
+  y.loss = s->loss.p;
+  sgemm<0, 0, mlp::EPI_MSE>(y, st);
+  auto weights = [&](int l, const float* A, const int* arows, const float* d) {
+    const int M = l ? h : s->n_in, N = l < 3 ? h : s->n_out;
+    mlp::GemmArgs g = gemm_args(M, N, B, A, d, s->red.p + t.base[l]);
+    g.rows = arows;
+    g.kchunk = slice_chunk(M, N, B);
+    sgemm<1, 0, mlp::EPI_SLICE>(g, st);
+  };
+  auto back = [&](int l, const float* d, float* Z, float* out) {  // through layer l to the pre-activations before it
+    mlp::GemmArgs g = gemm_args(B, h, l < 3 ? h : s->n_out, d, P(s, 2 * l), out);
+    g.aux = Z;
+    sgemm<0, 1, mlp::EPI_GELU_BWD>(g, st);
+  };
+  weights(3, s->A3.p, nullptr, s->dY.p);
+  back(3, s->dY.p, s->Z3.p, s->dZ.p);
+  weights(2, s->A2.p, nullptr, s->dZ.p);
+  back(2, s->dZ.p, s->Z2.p, s->dA.p);
+  weights(1, s->A1.p, nullptr, s->dA.p);
+  back(1, s->dA.p, s->Z1.p, s->dZ.p);
+  weights(0, X, rows, s->dZ.p);
+  return cudaGetLastError();
 }
 
 // Inference with ping-pong activations a0, a1 (rows x h each).
 void seed_forward_infer(adg_seed* s, const float* X, int B, float* a0, float* a1, float* Y, cudaStream_t st) {
-  using namespace mlp;
-  sgemm(0, 0, B, s->h, s->n_in, X, P(s, 0), a0, P(s, 1), nullptr, EPI_BIAS_GELU, st);
-  sgemm(0, 0, B, s->h, s->h, a0, P(s, 2), a1, P(s, 3), nullptr, EPI_BIAS_GELU, st);
-  sgemm(0, 0, B, s->h, s->h, a1, P(s, 4), a0, P(s, 5), nullptr, EPI_BIAS_GELU, st);
-  sgemm(0, 0, B, s->n_out, s->h, a0, P(s, 6), Y, P(s, 7), nullptr, EPI_BIAS, st);
+  forward_layer(s, 0, B, X, nullptr, nullptr, a0, st);
+  forward_layer(s, 1, B, a0, nullptr, nullptr, a1, st);
+  forward_layer(s, 2, B, a1, nullptr, nullptr, a0, st);
+  forward_layer(s, 3, B, a0, nullptr, nullptr, Y, st);
 }
 
 cudaError_t grow_rows(DevBuf<float>& b, size_t keep, size_t need) {
@@ -2872,7 +2905,6 @@ int adg_seed_train(adg_seed* s, int epochs, int batch, double lr, double* last_l
   if (seed_work(s, batch) != cudaSuccess || s->idx.ensure(s->nsamp) != cudaSuccess) return ADG_ERR_CUDA;
   std::vector<int> perm(s->nsamp);
   for (long long i = 0; i < s->nsamp; ++i) perm[i] = (int)i;
-  double epoch_loss = 0.0;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   for (int ep = 0; ep < epochs; ++ep) {
     std::shuffle(perm.begin(), perm.end(), s->rng);
@@ -2880,25 +2912,19 @@ int adg_seed_train(adg_seed* s, int epochs, int batch, double lr, double* last_l
     cudaMemsetAsync(s->loss.p, 0, sizeof(double), s->stream);
     for (long long b0 = 0; b0 < s->nsamp; b0 += batch) {
       const int B = (int)std::min<long long>(batch, s->nsamp - b0);
-      mlp::k_gather_rows<<<(unsigned)(((long long)B * s->n_in + 255) / 256), 256, 0, s->stream>>>(
-          B, s->n_in, s->idx.p + b0, s->X.p, s->Xb.p);
-      mlp::k_gather_rows<<<(unsigned)(((long long)B * s->n_out + 255) / 256), 256, 0, s->stream>>>(
-          B, s->n_out, s->idx.p + b0, s->T.p, s->Tb.p);
-      seed_forward_train(s, s->Xb.p, B, s->stream);
-      mlp::k_mse_grad<<<(unsigned)(((long long)B * s->n_out + 255) / 256), 256, 0, s->stream>>>(
-          B, s->n_out, s->Y.p, s->Tb.p, s->dY.p, s->loss.p);
-      seed_backward(s, s->Xb.p, B, s->stream);
+      if (seed_pass(s, s->X.p, s->T.p, s->idx.p + b0, B, s->stream) != cudaSuccess) return ADG_ERR_CUDA;
       s->adam_t++;
       const float bc1 = 1.f - (float)std::pow(b1, (double)s->adam_t), bc2 = 1.f - (float)std::pow(b2, (double)s->adam_t);
-      mlp::k_adam<<<(unsigned)((s->nparam + 255) / 256), 256, 0, s->stream>>>((int)s->nparam, s->params.p, s->grads.p,
-                                                                              s->am.p, s->av.p, (float)lr, b1, b2, eps,
-                                                                              bc1, bc2);
+      mlp::k_adam<<<(unsigned)((s->nparam + 31) / 32), dim3(32, mlp::kSliceRows), 0, s->stream>>>(
+          (int)s->nparam, s->params.p, slice_tab(s, B), s->red.p, s->am.p, s->av.p, (float)lr, b1, b2, eps, bc1, bc2);
     }
-    double l = 0.0;
-    cudaMemcpyAsync(&l, s->loss.p, sizeof(double), cudaMemcpyDeviceToHost, s->stream);
-    if (cudaStreamSynchronize(s->stream) != cudaSuccess) return ADG_ERR_CUDA;
-    epoch_loss = l / ((double)s->nsamp * s->n_out);
   }
+  // (one wait at the end: the next epoch's order is drawn while this one runs)
+  double l = 0.0;
+  if (epochs > 0)
+    cudaMemcpyAsync(&l, s->loss.p, sizeof(double), cudaMemcpyDeviceToHost, s->stream);
+  if (cudaStreamSynchronize(s->stream) != cudaSuccess) return ADG_ERR_CUDA;
+  const double epoch_loss = epochs > 0 ? l / ((double)s->nsamp * s->n_out) : 0.0;
   if (last_loss) *last_loss = epoch_loss;
   return seed_pack_tc(s);
 }
@@ -2919,14 +2945,15 @@ int adg_seed_forward(adg_seed* s, const float* X, int n, float* Y) {
 
 int adg_seed_gradients(adg_seed* s, const float* X, const float* T, int n, float* grads, double* loss) {
   if (!s || !X || !T || !grads || n <= 0) return ADG_ERR_ARG;
-  if (seed_work(s, n) != cudaSuccess) return ADG_ERR_CUDA;
+  if (seed_work(s, n) != cudaSuccess || s->Xb.ensure((size_t)n * s->n_in) != cudaSuccess ||
+      s->Tb.ensure((size_t)n * s->n_out) != cudaSuccess)
+    return ADG_ERR_CUDA;
   cudaMemcpyAsync(s->Xb.p, X, (size_t)n * s->n_in * 4, cudaMemcpyHostToDevice, s->stream);
   cudaMemcpyAsync(s->Tb.p, T, (size_t)n * s->n_out * 4, cudaMemcpyHostToDevice, s->stream);
   cudaMemsetAsync(s->loss.p, 0, sizeof(double), s->stream);
-  seed_forward_train(s, s->Xb.p, n, s->stream);
-  mlp::k_mse_grad<<<(unsigned)(((long long)n * s->n_out + 255) / 256), 256, 0, s->stream>>>(n, s->n_out, s->Y.p,
-                                                                                          s->Tb.p, s->dY.p, s->loss.p);
-  seed_backward(s, s->Xb.p, n, s->stream);
+  if (seed_pass(s, s->Xb.p, s->Tb.p, nullptr, n, s->stream) != cudaSuccess) return ADG_ERR_CUDA;
+  mlp::k_sum_slices<<<(unsigned)((s->nparam + 31) / 32), dim3(32, mlp::kSliceRows), 0, s->stream>>>(
+      (int)s->nparam, slice_tab(s, n), s->red.p, s->grads.p);
   double l = 0.0;
   cudaMemcpyAsync(&l, s->loss.p, sizeof(double), cudaMemcpyDeviceToHost, s->stream);
   cudaMemcpyAsync(grads, s->grads.p, s->nparam * 4, cudaMemcpyDeviceToHost, s->stream);

@@ -383,3 +383,28 @@ def test_seeded_run_stays_close_to_plain_run(mode):
         scale = np.max(np.abs(ua[:, 0 if q == 2 else q, 0]))
         assert np.max(np.abs(ub[:, q] - ua[:, q])) < 1e-5 * scale, q
     assert b.status() == 0
+
+
+@pytest.mark.parametrize("hidden,n", [(1, 1), (33, 17), (64, 63), (96, 64), (100, 129), (128, 1000), (128, 8229), (130, 20001)])
+def test_gradients_at_tile_edges(hidden, n):
+    """Both tile widths, ragged rows, columns and splits, strides that are not
+    multiples of four.  An output is one chain of at most 130 FMAs a layer and
+    the gradients one of a slice and its sum (at most 160 + 160): seven such
+    chains lie behind one another, 7 * 320 * 2^-24 = 1.3e-4 of the sums of the
+    terms' magnitudes, which the activations' derivatives (at most 1.13) keep."""
+    s = G.PredictorSeed(2, 1, hidden=hidden, rng_seed=3)
+    r = np.random.default_rng(hidden + n)
+    X = r.standard_normal((n, s.n_in)).astype(np.float32)
+    T = r.standard_normal((n, s.n_out)).astype(np.float32)
+    g, loss = s.gradients(X, T)
+    layers = _layers64(s)
+    lr, gr = mlp_ref.loss_and_grads(layers, X.astype(np.float64), T.astype(np.float64))
+    assert abs(loss - lr) < 1.3e-4 * lr
+    Y, acts, zs = mlp_ref.forward(layers, X.astype(np.float64))
+    d = 2.0 * np.abs(Y - T) / Y.size + 1.3e-4 * np.max(np.abs(Y)) / Y.size
+    bound = [None] * 4
+    for i in range(3, -1, -1):
+        bound[i] = (np.abs(acts[i]).T @ d, d.sum(axis=0))
+        d = (d @ np.abs(layers[i][0]).T) * 1.13
+    err = np.abs(g - mlp_ref.flatten(gr))
+    assert np.all(err <= 1.3e-4 * mlp_ref.flatten(bound) + 1e-12)
