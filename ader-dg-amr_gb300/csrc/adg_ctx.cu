@@ -131,6 +131,7 @@ struct adg_ctx {
   long long launches = 0;
 
   Hierarchy hier;       // host layout (levels, boxes, element and face tables)
+  Hierarchy hier_next;  // the layout being built by a regrid, then the previous one: its memory is reused
   amr::GridParams gp;
   bool initialised = false;
   bool tables_dirty = true;
@@ -297,6 +298,10 @@ LevelGeom level_geom(const adg_ctx* ctx) {
 struct RemapTable {
   std::vector<int> dst, par, src;
   std::vector<int8_t> ch;
+  void resize(size_t n) {
+    for (auto* v : {&dst, &par, &src}) v->resize(n);
+    ch.resize(n);
+  }
 };
 
 int upload_tables(adg_ctx* ctx, const RemapTable* rm = nullptr) {
@@ -371,27 +376,34 @@ int upload_tables(adg_ctx* ctx, const RemapTable* rm = nullptr) {
   {
     const size_t nv = H.n_valid(), ne = H.n_elem(), nf = H.face_left.size();
     const size_t nov1 = ((size_t)1 << D) + 1;
-    std::vector<uint8_t> covered(ne, 0);
-    for (size_t r = 0; r + nov1 <= ad.size(); r += nov1) covered[ad[r]] = 1;
     if (ad.size() >= nov1) {
       std::vector<uint8_t> fneed(nf, 0), eneed(ne, 0);
-      auto uncovered = [&](int e) { return (size_t)e < nv && !covered[e]; };
-      for (size_t f = 0; f < nf; ++f)
-        if (uncovered(H.face_left[f]) || uncovered(H.face_right[f])) fneed[f] = 1;
+      std::vector<uint8_t> open(ne, 0);  // uncovered valid elements
+      for (size_t e = 0; e < nv; ++e) open[e] = !H.cov[e];
+      for (size_t f = 0; f < nf; ++f) fneed[f] = open[H.face_left[f]] | open[H.face_right[f]];
       for (int f : H.rf_face) fneed[f] = 1;
       for (int f : H.rf_fine) fneed[f] = 1;
+      face_l.resize(nf);
+      size_t n = 0;
       for (size_t f = 0; f < nf; ++f)
         if (fneed[f]) {
-          face_l.push_back((int)f);
+          face_l[n++] = (int)f;
           eneed[H.face_left[f]] = eneed[H.face_right[f]] = 1;
         }
+      face_l.resize(n);
+      corr_l.resize(nv);
+      n = 0;
       for (size_t e = 0; e < nv; ++e)
-        if (!covered[e]) {
+        if (open[e]) {
           eneed[e] = 1;
-          if (roe[e] < 0) corr_l.push_back((int)e);
+          if (roe[e] < 0) corr_l[n++] = (int)e;
         }
+      corr_l.resize(n);
+      pred_l.resize(ne);
+      n = 0;
       for (size_t e = 0; e < ne; ++e)
-        if (eneed[e]) pred_l.push_back((int)e);
+        if (eneed[e]) pred_l[n++] = (int)e;
+      pred_l.resize(n);
     }
   }
   ctx->n_pred = pred_l.size();
@@ -400,17 +412,20 @@ int upload_tables(adg_ctx* ctx, const RemapTable* rm = nullptr) {
   add(ctx->pred_list, pred_l);
   add(ctx->face_list, face_l);
   add(ctx->corr_list, corr_l);
-  // ghost fills grouped by child index: the warps of the fill kernel then
-  // mostly run a single coarse-to-fine operator
-  std::vector<size_t> gperm(H.gf_elem.size());
-  for (size_t i = 0; i < gperm.size(); ++i) gperm[i] = i;
-  std::stable_sort(gperm.begin(), gperm.end(), [&](size_t x, size_t y) { return H.gf_child[x] < H.gf_child[y]; });
-  std::vector<int> gfe(gperm.size()), gfp(gperm.size());
-  std::vector<int8_t> gfc(gperm.size());
-  for (size_t i = 0; i < gperm.size(); ++i) {
-    gfe[i] = H.gf_elem[gperm[i]];
-    gfp[i] = H.gf_parent[gperm[i]];
-    gfc[i] = H.gf_child[gperm[i]];
+  // ghost fills grouped by child index, in order within it
+  const size_t ng = H.gf_elem.size();
+  std::vector<int> gfe(ng), gfp(ng);
+  std::vector<int8_t> gfc(ng);
+  {
+    size_t at[9] = {};
+    for (int8_t c : H.gf_child) ++at[c + 1];
+    for (int c = 0; c < 8; ++c) at[c + 1] += at[c];
+    for (size_t i = 0; i < ng; ++i) {
+      const size_t to = at[H.gf_child[i]]++;
+      gfe[to] = H.gf_elem[i];
+      gfp[to] = H.gf_parent[i];
+      gfc[to] = H.gf_child[i];
+    }
   }
   add(ctx->gf_elem, gfe);
   add(ctx->gf_parent, gfp);
@@ -919,7 +934,7 @@ int apply_layout(adg_ctx* ctx, const std::vector<std::vector<amr::IBox>>& ng,
                  std::chrono::steady_clock::time_point t2) {
   Hierarchy& H = ctx->hier;
   const KernelSet* ks = ctx->ks;
-  Hierarchy NH;
+  Hierarchy& NH = ctx->hier_next;
   std::string msg;
   if (!NH.build(ctx->gp, ng, ctx->cfg.reflux_box_quirk, &msg, !ctx->cfg.no_reflux))
     return fail(ctx, ADG_ERR_LAYOUT, "layout: " + msg);
@@ -931,11 +946,12 @@ int apply_layout(adg_ctx* ctx, const std::vector<std::vector<amr::IBox>>& ng,
   ADG_CUDA(cudaMemcpyAsync(nU, ctx->Uw.p, H.level_valid_count(0) * Q * Ns * sizeof(double), cudaMemcpyDeviceToDevice,
                            ctx->stream), "regrid copy level 0");
   RemapTable rm;
+  rm.resize(NH.n_elem() - NH.level_valid_count(0));
   std::vector<size_t> lo(NH.nlevels() + 1, 0);
+  size_t nr = 0;
   for (int l = 1; l < NH.nlevels(); ++l) {
-    lo[l] = rm.dst.size();
-    for (size_t e = 0; e < NH.n_elem(); ++e) {
-      if (NH.elem_level[e] != l) continue;
+    lo[l] = nr;
+    auto add = [&](size_t e) {
       const int* c = &NH.elem_cell[3 * e];
       int pc[3] = {0, 0, 0}, child = 0;
       for (int a = 0; a < NH.D; ++a) {
@@ -944,20 +960,23 @@ int apply_layout(adg_ctx* ctx, const std::vector<std::vector<amr::IBox>>& ng,
       }
       int old = -1;
       if (l < H.nlevels()) {
-        int oe = H.elem_at(l, c);
+        const int oe = H.cellmap[l][H.cidx(l, c)];
         if (H.is_valid_elem(oe)) old = oe;
       }
-      rm.dst.push_back((int)e);
-      rm.par.push_back(NH.cellmap[l - 1][NH.cidx(l - 1, pc)]);
-      rm.src.push_back(old);
-      rm.ch.push_back((int8_t)child);
-    }
+      rm.dst[nr] = (int)e;
+      rm.par[nr] = NH.cellmap[l - 1][NH.cidx(l - 1, pc)];
+      rm.src[nr] = old;
+      rm.ch[nr++] = (int8_t)child;
+    };
+    const size_t e0 = NH.level_valid_offset(l), e1 = e0 + NH.level_valid_count(l);
+    for (size_t e = e0; e < e1; ++e) add(e);
+    for (size_t e = NH.n_valid(); e < NH.n_elem(); ++e)  // ghosts
+      if (NH.elem_level[e] == l) add(e);
   }
-  lo[NH.nlevels()] = rm.dst.size();
-  const size_t nr = rm.dst.size();
+  lo[NH.nlevels()] = nr;
   auto t3 = std::chrono::steady_clock::now();
   ctx->rg_phase_ms[2] += ms_between(t2, t3);
-  ctx->hier = std::move(NH);
+  std::swap(ctx->hier, ctx->hier_next);
   int rc = upload_tables(ctx, &rm);
   if (rc) return rc;
   auto t4 = std::chrono::steady_clock::now();
