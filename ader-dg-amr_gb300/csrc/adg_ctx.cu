@@ -2719,6 +2719,11 @@ int launch_seeded_predictor(adg_ctx* ctx, const PredictorArgs& base, cudaEvent_t
   // per SM, so the element groups spread evenly over the SMs (at D = 3 the
   // 40-thread blocks of 8 elements idle 3/8 of their lanes: the tuned E stays)
   const int Es = ctx->Es > 0 ? ctx->Es : (ctx->seed_mode == 2 && ctx->cfg.D == 2 ? 8 : ctx->E);
+  if (ctx->seed_mode == 2) {
+    e = ks->split_base(pa, st);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "time-independent part");
+    ctx->launches++;
+  }
   e = ks->predictor(pa, Es, st, ctx->seed_mode);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "seeded predictor");
   if (ev) cudaEventRecord(ev[7], st);  // end of the seeded predictor, start of the fallback pass

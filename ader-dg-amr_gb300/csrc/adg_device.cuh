@@ -7,6 +7,24 @@
 
 namespace adg {
 
+// Conversions between double and float, rounded to nearest even, in integer
+// code where both are normal numbers or zero: a hardware conversion occupies
+// the FP64 pipe (1.6 a clock and SM).
+__device__ __forceinline__ float to_float(double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const int mag = hi & 0x7fffffff;
+  if ((unsigned)(mag - (897 << 20)) >= (253u << 20)) return (mag | lo) == 0 ? __int_as_float(hi) : (float)x;
+  unsigned f = ((unsigned)(mag - (896 << 20)) << 3) | ((unsigned)lo >> 29);
+  const unsigned rest = (unsigned)lo << 3;  // the dropped bits, a half is 2^31
+  f += rest > 0x80000000u || (rest == 0x80000000u && (f & 1u));
+  return __int_as_float((int)(f | ((unsigned)hi & 0x80000000u)));
+}
+__device__ __forceinline__ double to_double(float x) {
+  const int f = __float_as_int(x), mag = f & 0x7fffffff;
+  if ((unsigned)(mag - 0x00800000) >= 0x7f000000u) return mag == 0 ? __hiloint2double(f, 0) : (double)x;
+  return __hiloint2double((f & (int)0x80000000) | ((mag >> 3) + (896 << 20)), f << 29);
+}
+
 // Operand accessors: the generated operators are written against these, so
 // the same code reads registers (stride 1, compile-time indices) or a shared
 // memory column (runtime stride).

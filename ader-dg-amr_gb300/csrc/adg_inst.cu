@@ -23,7 +23,7 @@ constexpr size_t smem_bytes() {
   constexpr size_t ld = E * O::Q + 1;
   constexpr bool split = MODE == 2 || MODE == 3;
   constexpr size_t sweeps = MODE == 2 ? O::D * O::NQ_S * ld * sizeof(float) : O::D * O::NQ_ST * ld * sizeof(double);
-  constexpr size_t fin = split ? split_epilogue_doubles<O>(ld) * sizeof(double)
+  constexpr size_t fin = split ? split_epilogue_doubles<O>(ld, MODE == 3) * sizeof(double)
                                : (1 + O::D) * O::NQ_S * ld * sizeof(double);
   constexpr size_t faces = split ? 0 : 2 * O::NQ_BD * ld * sizeof(double);
   constexpr size_t red = 2 * E * O::Q * sizeof(double);
@@ -75,6 +75,18 @@ cudaError_t launch_plain(const PredictorArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     k_predictor_fx<O, E><<<(a.n_elem + E - 1) / E, FxShape<O, E>::NT, smem, s>>>(a);
   }
+  return cudaGetLastError();
+}
+
+// The time-independent part of mode 2's final stage.
+template <int E>
+cudaError_t launch_split_base(const PredictorArgs& a, cudaStream_t s) {
+  constexpr size_t smem = FxBase<O, E>::BYTES;
+  static std::atomic<unsigned long long> attr{0};
+  if (a.n_elem <= 0) return cudaSuccess;
+  cudaError_t e = ensure_smem_attr(attr, k_split_base<O, E>, smem);
+  if (e != cudaSuccess) return e;
+  k_split_base<O, E><<<(a.n_elem + E - 1) / E, FxShape<O, E>::NT, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -169,6 +181,12 @@ struct Impl final : KernelSet {
     return launch_predictor<16>(a, s, mode);
   }
 #endif
+  cudaError_t split_base(const PredictorArgs& a, cudaStream_t s) const override {
+    if constexpr (kSeedModes) {
+      return launch_split_base<O::D == 2 ? 8 : 6>(a, s);
+    }
+    return cudaErrorNotSupported;
+  }
   cudaError_t numflux(const FaceArgs& a, long long nface, cudaStream_t s, bool split) const override {
     if (nface <= 0) return cudaSuccess;
     constexpr int FB = numflux_faces_per_block<O>();

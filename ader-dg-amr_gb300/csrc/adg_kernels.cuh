@@ -309,16 +309,19 @@ __device__ __forceinline__ void face_traces(const double* hw, double* sm, int co
 // the volume term (Rvol), and kept apart in the split trace tiles (U and
 // f_n(U) in FP64, the changes of u and f_n and the wave speed in FP32) that
 // k_numflux_split reads.
+// BASE: all of it (the fallback elements); else the time-independent part is
+// there already, in Rvol and the tiles (k_split_base of adg_predictor_fx.cuh).
 // ---------------------------------------------------------------------------
 
-// Shared memory of split_epilogue (doubles): region A = D NS ld doubles (U,
-// then F(U) at the spatial points; later the FP32 delta slice and flux
-// change sums; later the face buffers), then NS ld floats of U in FP32.
+// Shared memory of split_epilogue (doubles).  BASE: D NS ld doubles (U, then
+// F(U) at the spatial points; later the FP32 delta slice and flux change
+// sums), then NS ld floats of U in FP32; else D + 1 such slabs of floats and
+// U's.  Then the face buffers.
 template <class O>
-constexpr size_t split_epilogue_doubles(size_t ld) {
+constexpr size_t split_epilogue_doubles(size_t ld, bool base) {
   constexpr size_t NS = O::NQ_S, NB = O::NQ_BD, NSB = NB / O::N;
-  const size_t vol = O::D * NS * ld + (NS * ld + 1) / 2;
-  const size_t faces = (2 * NSB + (2 * NSB + 2 * NB + 1) / 2) * ld;
+  const size_t vol = base ? O::D * NS * ld + (NS * ld + 1) / 2 : ((O::D + 2) * NS * ld + 1) / 2;
+  const size_t faces = ((base ? 2 * NSB : 0) + (2 * NSB + 2 * NB + 1) / 2) * ld;
   return vol > faces ? vol : faces;
 }
 
@@ -358,20 +361,27 @@ __device__ __forceinline__ void delta_slices(const float* dlt, const float* us32
 // Column part of one face side: U at the face's spatial points (FP64) and
 // delta at its space-time points (FP32), to shared memory and to the split
 // trace tile (u_q and its change).
-template <class O, int E, int DIR, int S>
+template <class O, int E, bool BASE, int DIR, int S>
 __device__ __forceinline__ void split_face_column(const double* u, const float* dlt, double* uface64, float* uf32,
                                                   float* dface32, int col, int q, double* tr_elem) {
   constexpr int N = O::N, NB = O::NQ_BD, NSB = NB / N, LD = E * O::Q + 1, TT = tr_tile<O>();
   double uf[NSB];
   float df[NB];
-  O::template face_eval_sp<DIR, S>(RegIn{u}, RegOut{uf});
-  O::template face_eval<DIR, S, float>(RegInT<float>{dlt}, RegOutT<float>{df});  // point x N + t
   double* t = tr_elem ? tr_elem + (2 * DIR + S) * TT : nullptr;
+  if constexpr (BASE) {
+    O::template face_eval_sp<DIR, S>(RegIn{u}, RegOut{uf});
+  } else {
+#pragma unroll
+    for (int x = 0; x < NSB; ++x) uf[x] = t ? t[q * NSB + x] : 0.0;
+  }
+  O::template face_eval<DIR, S, float>(RegInT<float>{dlt}, RegOutT<float>{df});  // point x N + t
 #pragma unroll
   for (int x = 0; x < NSB; ++x) {
-    uface64[(S * NSB + x) * LD + col] = uf[x];
-    uf32[(S * NSB + x) * LD + col] = (float)uf[x];
-    if (t) t[q * NSB + x] = uf[x];
+    uf32[(S * NSB + x) * LD + col] = BASE ? (float)uf[x] : to_float(uf[x]);
+    if constexpr (BASE) {
+      uface64[(S * NSB + x) * LD + col] = uf[x];
+      if (t) t[q * NSB + x] = uf[x];
+    }
   }
   float* tf = t ? reinterpret_cast<float*>(t) + split_tr_float_off<O>() + q * NB : nullptr;
 #pragma unroll
@@ -388,19 +398,19 @@ __device__ __forceinline__ void split_face_column(const double* u, const float* 
 // The two faces of direction DIR as split trace tiles: u and its change
 // (columns), then f_n(u) at the faces' spatial points (FP64) and, per
 // space-time face point, the change of f_n and the wave speed (FP32).
-template <class O, int E, int DIR>
+template <class O, int E, bool BASE, int DIR>
 __device__ __forceinline__ void split_faces(const double* u, const float* dlt, double* sm, int col, int q,
                                             double* tr_elem, const PredictorArgs& a, int e0, int limit) {
   constexpr int D = O::D, Q = O::Q, N = O::N, NB = O::NQ_BD, NSB = NB / N, NF = 2 * D, TT = tr_tile<O>();
   constexpr int LD = E * Q + 1, FO = split_tr_float_off<O>();
   static_assert(split_tr_fits<O>(), "split trace tile larger than the FP64 tile");
   double* uface64 = sm;                                         // [side][x][col]
-  float* uf32 = reinterpret_cast<float*>(sm + 2 * NSB * LD);    // [side][x][col]
+  float* uf32 = reinterpret_cast<float*>(sm + (BASE ? 2 * NSB * LD : 0));  // [side][x][col]
   float* dface32 = uf32 + 2 * NSB * LD;                         // [side][t NSB + x][col]
-  split_face_column<O, E, DIR, 0>(u, dlt, uface64, uf32, dface32, col, q, tr_elem);
-  split_face_column<O, E, DIR, 1>(u, dlt, uface64, uf32, dface32, col, q, tr_elem);
+  split_face_column<O, E, BASE, DIR, 0>(u, dlt, uface64, uf32, dface32, col, q, tr_elem);
+  split_face_column<O, E, BASE, DIR, 1>(u, dlt, uface64, uf32, dface32, col, q, tr_elem);
   __syncthreads();
-  for (int it = threadIdx.x; it < E * 2 * NSB; it += blockDim.x) {
+  for (int it = threadIdx.x; BASE && it < E * 2 * NSB; it += blockDim.x) {
     const int x = it % NSB;
     const int s = (it / NSB) & 1;
     const int ee = it / (2 * NSB);
@@ -439,7 +449,7 @@ __device__ __forceinline__ void split_faces(const double* u, const float* dlt, d
   __syncthreads();
 }
 
-template <class O, int E>
+template <class O, int E, bool BASE>
 __device__ __forceinline__ void split_epilogue(const double* u, const float* uf, const float* dlt, const double* c,
                                                double gm1, double* sm, int col, int q, bool live, int e, int e0,
                                                int limit, const PredictorArgs& a) {
@@ -447,33 +457,36 @@ __device__ __forceinline__ void split_epilogue(const double* u, const float* uf,
   constexpr int LD = E * Q + 1;
   double* us64 = sm;  // U, then F_0(U) in place
   double* fU64 = sm;  // F_d(U) in slab d
-  float* us32 = reinterpret_cast<float*>(sm + D * NS * LD);
+  float* us32 = BASE ? reinterpret_cast<float*>(sm + D * NS * LD) : reinterpret_cast<float*>(sm) + (D + 1) * NS * LD;
 
   // U at the spatial points (FP64, and in FP32 from the FP32 modes uf for
   // the flux changes)
-  O::sp_eval(RegIn{u}, ColOut{us64 + col, LD});
+  if constexpr (BASE) O::sp_eval(RegIn{u}, ColOut{us64 + col, LD});
   O::template sp_eval<float>(RegInT<float>{uf}, ColOutT<float>{us32 + col, LD});
   __syncthreads();
-  // F(U) at the spatial points (FP64)
-  flux_stage<O, E, NS, double>(us64, LD, gm1);
-  __syncthreads();
-  // volume term of the time-constant part (AmrDG.tpp:696-709 with F = F(U)):
-  // M U + sum_d c_d (sum_k w_k) Sk_d F_d(U)
-  double R[NP_S], v[NP_S];
+  double R[NP_S];
+  if constexpr (BASE) {
+    // F(U) at the spatial points (FP64)
+    flux_stage<O, E, NS, double>(us64, LD, gm1);
+    __syncthreads();
+    // volume term of the time-constant part (AmrDG.tpp:696-709 with F = F(U)):
+    // M U + sum_d c_d (sum_k w_k) Sk_d F_d(U)
+    double v[NP_S];
 #pragma unroll
-  for (int n = 0; n < NP_S; ++n) R[n] = O::mdiag(n) * u[n];
-  O::template vol_term_sp<0>(ColIn{fU64 + col, LD}, RegOut{v});
+    for (int n = 0; n < NP_S; ++n) R[n] = O::mdiag(n) * u[n];
+    O::template vol_term_sp<0>(ColIn{fU64 + col, LD}, RegOut{v});
 #pragma unroll
-  for (int n = 0; n < NP_S; ++n) R[n] = fma(c[0] * O::WEIGHT_SUM, v[n], R[n]);
-  O::template vol_term_sp<1>(ColIn{fU64 + NS * LD + col, LD}, RegOut{v});
+    for (int n = 0; n < NP_S; ++n) R[n] = fma(c[0] * O::WEIGHT_SUM, v[n], R[n]);
+    O::template vol_term_sp<1>(ColIn{fU64 + NS * LD + col, LD}, RegOut{v});
 #pragma unroll
-  for (int n = 0; n < NP_S; ++n) R[n] = fma(c[1] * O::WEIGHT_SUM, v[n], R[n]);
-  if constexpr (D == 3) {
-    O::template vol_term_sp<2>(ColIn{fU64 + 2 * NS * LD + col, LD}, RegOut{v});
+    for (int n = 0; n < NP_S; ++n) R[n] = fma(c[1] * O::WEIGHT_SUM, v[n], R[n]);
+    if constexpr (D == 3) {
+      O::template vol_term_sp<2>(ColIn{fU64 + 2 * NS * LD + col, LD}, RegOut{v});
 #pragma unroll
-    for (int n = 0; n < NP_S; ++n) R[n] = fma(c[2] * O::WEIGHT_SUM, v[n], R[n]);
+      for (int n = 0; n < NP_S; ++n) R[n] = fma(c[2] * O::WEIGHT_SUM, v[n], R[n]);
+    }
+    __syncthreads();
   }
-  __syncthreads();
   // time-dependent part: the time integrals of the flux changes (FP32)
   float* ds32 = reinterpret_cast<float*>(sm);
   float* fb32 = ds32 + NS * LD;
@@ -491,8 +504,13 @@ __device__ __forceinline__ void split_epilogue(const double* u, const float* uf,
 #pragma unroll
       for (int n = 0; n < NP_S; ++n) ws[n] = fmaf((float)c[2], w[n], ws[n]);
     }
+    if constexpr (!BASE) {
+      const double* src = a.Rvol + ((size_t)e * Q + q) * NP_S;
 #pragma unroll
-    for (int n = 0; n < NP_S; ++n) R[n] += (double)ws[n];
+      for (int n = 0; n < NP_S; ++n) R[n] = live ? src[n] : 0.0;
+    }
+#pragma unroll
+    for (int n = 0; n < NP_S; ++n) R[n] += BASE ? (double)ws[n] : to_double(ws[n]);
   }
   if (live) {
     double* dst = a.Rvol + ((size_t)e * Q + q) * NP_S;
@@ -502,9 +520,9 @@ __device__ __forceinline__ void split_epilogue(const double* u, const float* uf,
   __syncthreads();
   // face traces, one direction at a time
   double* tr_elem = live ? a.Tr + (size_t)e * NF * tr_tile<O>() : nullptr;
-  split_faces<O, E, 0>(u, dlt, sm, col, q, tr_elem, a, e0, limit);
-  split_faces<O, E, 1>(u, dlt, sm, col, q, tr_elem, a, e0, limit);
-  if constexpr (D == 3) split_faces<O, E, 2>(u, dlt, sm, col, q, tr_elem, a, e0, limit);
+  split_faces<O, E, BASE, 0>(u, dlt, sm, col, q, tr_elem, a, e0, limit);
+  split_faces<O, E, BASE, 1>(u, dlt, sm, col, q, tr_elem, a, e0, limit);
+  if constexpr (D == 3) split_faces<O, E, BASE, 2>(u, dlt, sm, col, q, tr_elem, a, e0, limit);
 }
 
 // Final stage of the FP64 paths: the corrector volume term and the face
@@ -557,7 +575,8 @@ __device__ __forceinline__ void fp64_epilogue(const double* hw, const double* u,
 // of MODE 2 (the fallback elements of a MODE 2 step).
 // (Mode 0, the plain path, is k_predictor_fx of adg_predictor_fx.cuh.)
 // Resident blocks per SM that MODE 2 asks for: 16 warps (at most 128
-// registers a thread); its sliced sweeps leave the shared memory for them.
+// registers a thread); its sliced sweeps leave the shared memory for them
+// (D2P3, 15,600 elements, 16 / 20 / 24 / 32 warps: 45 / 47 / 48 / 51 us).
 template <int E, int Q, int MODE>
 constexpr int predictor_min_blocks() {
   constexpr int warps = (E * Q + 31) / 32;
@@ -680,7 +699,7 @@ __device__ __forceinline__ void predictor_chunk(const PredictorArgs& a, double* 
         for (int n = 0; n < NP_ST; ++n) hf[n] = (float)a.Hseed[hoff + n];
       }
 #pragma unroll
-      for (int n = 0; n < NP_S; ++n) uf[n] = (float)u[n];
+      for (int n = 0; n < NP_S; ++n) uf[n] = to_float(u[n]);
       O::template wu<float>(RegInT<float>{uf}, RegOutT<float>{wf});
 #pragma unroll
       for (int d = 0; d < D; ++d) cf[d] = (float)c[d];
@@ -730,7 +749,7 @@ __device__ __forceinline__ void predictor_chunk(const PredictorArgs& a, double* 
 #pragma unroll
       for (int n = 0; n < NP_S; ++n) uf[n] = (float)u[n];
     }
-    split_epilogue<O, E>(u, uf, dlt, c, gm1, sm, col, q, live, e, e0, limit, a);
+    split_epilogue<O, E, MODE == 3>(u, uf, dlt, c, gm1, sm, col, q, live, e, e0, limit, a);
   } else {
     fp64_epilogue<O, E>(hw, u, c, gm1, sm, col, q, live, e, e0, limit, a);
   }

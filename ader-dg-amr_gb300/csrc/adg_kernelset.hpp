@@ -29,6 +29,9 @@ struct KernelSet {
   // fallback) is strided over by a short grid; one counted on the host
   // (a.list_count == nullptr, a.n_elem entries) runs one group per block.
   virtual cudaError_t predictor(const PredictorArgs& a, int E, cudaStream_t s, int mode = 0) const = 0;
+  // the time-independent part of mode 2's final stage, before that mode's
+  // launch on the same elements
+  virtual cudaError_t split_base(const PredictorArgs& a, cudaStream_t s) const = 0;
   // split: the trace tiles are split tiles (predictor modes 2 and 3);
   // nface: the faces computed (a.n_list with a face list)
   virtual cudaError_t numflux(const FaceArgs& a, long long nface, cudaStream_t s, bool split = false) const = 0;

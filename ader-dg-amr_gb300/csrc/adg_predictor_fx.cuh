@@ -353,30 +353,15 @@ __device__ __forceinline__ void fx_accumulate(const FxBlock<O, E>& kf, int kt) {
   }
 }
 
-// Phases 2 to 5 of one slice: H from the spatial modes g, fluxes, projections,
-// accumulation.  kt < 0: the first sweep's slice (g = U).  k: all columns, kf:
-// those projected.
-template <class O, int E>
-__device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxBlock<O, E>& kf, const long long* g,
-                                               const FxCoef* c1, const FxCoef* c2, int kt, double gm1,
-                                               const FxFactor& gm1x) {
+// Phase 3: the fluxes of the slice's points in the place of their values;
+// MASS: the momenta as the mass fluxes too.  An element with a point that is
+// not for the integers (or with exponents near the range of doubles) has all
+// of its points in FP64.  of_u: values of U, else of H.
+template <class O, int E, bool MASS>
+__device__ __forceinline__ void fx_point_fluxes(const FxBlock<O, E>& k, bool of_u, double gm1, const FxFactor& gm1x) {
   using S = FxShape<O, E>;
-  constexpr int D = O::D, Q = O::Q, N = O::N, P = O::P, LD = S::LD;
-  if (k.act) {
-    long long t[N];
-    fx_line_modes<O, LD>(g + k.col, c1, c2, t);
-    long long* h = k.m + S::O_F + k.line * LD + k.col;
-    int n = 0;
-    fx_line_points<O>(t, [&](int k0, long long v) {
-      h[k0 * S::LINES * LD] = v;
-      n = max(n, __clz((int)(v >> 32)));
-    });
-    if (k.col % Q == 0) atomicMax(&k.word(S::I_N), n);
-  }
-  fx_sync<S::NT>();
-  // fluxes; an element with a point that is not for the integers (or with
-  // exponents near the range of doubles) has all of its points in FP64
-  const int* wx = k.w + (kt < 0 ? S::I_EU : S::I_EH);
+  constexpr int D = O::D, Q = O::Q, LD = S::LD;
+  const int* wx = k.w + (of_u ? S::I_EU : S::I_EH);
   long long u[S::PTS][Q];
   bool bad = false;
 #pragma unroll
@@ -400,7 +385,7 @@ __device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxB
 #pragma unroll
         for (int d = 0; d < D; ++d)
 #pragma unroll
-          for (int v = 1; v < Q; ++v) base[d * S::NS * LD + v] = F[d][v - 1];
+          for (int v = MASS ? 0 : 1; v < Q; ++v) base[d * S::NS * LD + v] = v ? F[d][v > 0 ? v - 1 : 0] : u[r][d + 1];
       } else {
         k.w[S::I_F64 + c0] = 1;
         bad = true;
@@ -409,7 +394,7 @@ __device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxB
 #pragma unroll
         for (int d = 0; d < D; ++d)
 #pragma unroll
-          for (int v = 1; v < Q; ++v) k.w[S::I_X + d * S::C + c0 + v] = x.flux(d, v, em);
+          for (int v = MASS ? 0 : 1; v < Q; ++v) k.w[S::I_X + d * S::C + c0 + v] = v ? x.flux(d, v, em) : em[d];
       }
     }
   }
@@ -423,16 +408,40 @@ __device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxB
         double ud[Q], F[D * Q];
 #pragma unroll
         for (int v = 0; v < Q; ++v)
-          ud[v] = fx_to_double(u[r][v], wx[c0 + v], kt < 0 ? fx_poison(wx[c0 + v]) : k.w[S::I_NAN + c0 + v]);
+          ud[v] = fx_to_double(u[r][v], wx[c0 + v], of_u ? fx_poison(wx[c0 + v]) : k.w[S::I_NAN + c0 + v]);
         euler_flux_all<D, double>(ud, gm1, F);
 #pragma unroll
         for (int d = 0; d < D; ++d)
 #pragma unroll
-          for (int v = 1; v < Q; ++v) base[d * S::NS * LD + v] = F[d * Q + v];
+          for (int v = MASS ? 0 : 1; v < Q; ++v) base[d * S::NS * LD + v] = F[d * Q + v];
       }
     }
     fx_sync<S::NT>();
   }
+}
+
+// Phases 2 to 5 of one slice: H from the spatial modes g, fluxes, projections,
+// accumulation.  kt < 0: the first sweep's slice (g = U).  k: all columns, kf:
+// those projected.
+template <class O, int E>
+__device__ __forceinline__ void fx_sweep_slice(const FxBlock<O, E>& k, const FxBlock<O, E>& kf, const long long* g,
+                                               const FxCoef* c1, const FxCoef* c2, int kt, double gm1,
+                                               const FxFactor& gm1x) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D, Q = O::Q, N = O::N, P = O::P, LD = S::LD;
+  if (k.act) {
+    long long t[N];
+    fx_line_modes<O, LD>(g + k.col, c1, c2, t);
+    long long* h = k.m + S::O_F + k.line * LD + k.col;
+    int n = 0;
+    fx_line_points<O>(t, [&](int k0, long long v) {
+      h[k0 * S::LINES * LD] = v;
+      n = max(n, __clz((int)(v >> 32)));
+    });
+    if (k.col % Q == 0) atomicMax(&k.word(S::I_N), n);
+  }
+  fx_sync<S::NT>();
+  fx_point_fluxes<O, E, false>(k, kt < 0, gm1, gm1x);
   const bool f64 = kf.act && k.w[S::I_F64 + kf.col / Q * Q];
   if (kf.act) {
 #pragma unroll 1
@@ -621,30 +630,27 @@ __device__ __forceinline__ void fx_time_slice(const FxBlock<O, E>& k, const FxMo
 
 // Face values of a slice: the two faces of x_0 from the line's modes, the
 // others from lines that run along them (D = 2: the two sides of x_1; D = 3:
-// side and x_2, x_1 and side), written to the trace tiles (time node kt).
-template <class O, int E>
-__device__ __forceinline__ void fx_face_values(const FxBlock<O, E>& k, const long long* t, int eg, int nan_bits,
-                                               double* tr) {
-  constexpr int TT = tr_tile<O>();
+// side and x_2, x_1 and side): out(face 2d + side, point, value).
+template <class O, int E, class Out>
+__device__ __forceinline__ void fx_face_values(const FxBlock<O, E>& k, const long long* t, Out out) {
   long long lo = t[0], hi = t[0];
 #pragma unroll
   for (int n = 1; n <= O::P; ++n) {
     hi += t[n];
     lo += n % 2 ? -t[n] : t[n];
   }
-  tr[k.line] = fx_to_double(lo, eg, nan_bits);
-  tr[TT + k.line] = fx_to_double(hi, eg, nan_bits);
+  out(0, k.line, lo);
+  out(1, k.line, hi);
 }
 
-template <class O, int E>
-__device__ __forceinline__ void fx_side_lines(const FxBlock<O, E>& k, const long long* g, int eg, int nan_bits,
-                                              double* tr) {
+template <class O, int E, class Out>
+__device__ __forceinline__ void fx_side_lines(const FxBlock<O, E>& k, const long long* g, Out out) {
   using S = FxShape<O, E>;
-  constexpr int D = O::D, N = O::N, TT = tr_tile<O>(), SIDES = D == 2 ? 2 : 4 * N;
+  constexpr int D = O::D, N = O::N, SIDES = D == 2 ? 2 : 4 * N;
 #pragma unroll 1
   for (int i = k.line; i < SIDES; i += S::LINES) {
     FxCoef c1[N], c2[N];
-    int face, x;  // face 2d + side, point offset
+    int face, x;  // point offset
     if constexpr (D == 2) {
       fx_end_coefs<O>(i, c1);
       face = 2 + i;
@@ -663,8 +669,7 @@ __device__ __forceinline__ void fx_side_lines(const FxBlock<O, E>& k, const long
     }
     long long t[N];
     fx_line_modes<O, S::LD>(g + k.col, c1, c2, t);
-    double* out = tr + face * TT + x;
-    fx_line_points<O>(t, [&](int k0, long long v) { out[k0 * (D == 2 ? 1 : N)] = fx_to_double(v, eg, nan_bits); });
+    fx_line_points<O>(t, [&](int k0, long long v) { out(face, x + k0 * (D == 2 ? 1 : N), v); });
   }
 }
 
@@ -684,19 +689,22 @@ __device__ __forceinline__ void fx_volume_last(const FxBlock<O, E>& k, int pre) 
     if (n <= O::P - deg) out[n * S::LD] = fx_to_double(p.template row<TAB>(n), e, nan_bits);
 }
 
-template <class O, int E>
+// FX: the fluxes are those of fx_point_fluxes, else doubles.
+template <class O, int E, bool FX>
 __device__ __forceinline__ void fx_volume_term(const FxBlock<O, E>& k) {
   using S = FxShape<O, E>;
   constexpr int D = O::D;
+  const bool f64 = !FX || (k.act && k.w[S::I_F64 + k.col / O::Q * O::Q]);
+  auto exp = [&](int d) { return FX ? k.word(S::I_X, d) : 0; };
   if (k.act) {
 #pragma unroll 1
-    for (int d = 0; d < D; ++d) fx_line_max<O, E>(k, d, true, 0);
+    for (int d = 0; d < D; ++d) fx_line_max<O, E>(k, d, f64, exp(d));
   }
   fx_sync<S::NT>();
   if (k.act) {
-    fx_line_project<O, E, FX_D>(k, 0, fx_line_exp<O, E>(k, 0), true, 0);
+    fx_line_project<O, E, FX_D>(k, 0, fx_line_exp<O, E>(k, 0), f64, exp(0));
 #pragma unroll 1
-    for (int d = 1; d < D; ++d) fx_line_project<O, E, FX_W>(k, d, fx_line_exp<O, E>(k, d), true, 0);
+    for (int d = 1; d < D; ++d) fx_line_project<O, E, FX_W>(k, d, fx_line_exp<O, E>(k, d), f64, exp(d));
   }
   fx_sync<S::NT>();
   if constexpr (D == 3) {
@@ -718,6 +726,35 @@ __device__ __forceinline__ void fx_volume_term(const FxBlock<O, E>& k) {
         if (d == 2) fx_volume_last<O, E, 2>(k, pre);
     }
   }
+  fx_sync<S::NT>();
+}
+
+// U of the block's elements: coalesced loads, the column's exponent, fixed
+// point; the words' initial values.
+template <class O, int E, class Elem>
+__device__ __forceinline__ void fx_load_state(const FxBlock<O, E>& k, const PredictorArgs& a, Elem element, bool live) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D, Q = O::Q, NP_S = O::NP_S, LD = S::LD, C = S::C, NT = S::NT;
+  const int el = k.col / Q, q = k.col % Q;
+  double* ud = reinterpret_cast<double*>(k.m + S::O_G);
+  for (int i = threadIdx.x; i < C * NP_S; i += NT)
+    ud[(i % NP_S) * LD + i / NP_S] = a.Uw[(size_t)element(i / (Q * NP_S)) * Q * NP_S + i % (Q * NP_S)];
+  fx_sync<S::NT>();
+  if (k.act && k.line == 0) {
+    const int eu = fx_norm_exp<NP_S>(ud + k.col, LD);
+    k.word(S::I_EU) = eu;
+    k.word(S::I_SUM) = k.word(S::I_N) = k.word(S::I_F64) = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      k.word(S::I_Z, d) = 0;
+      k.word(S::I_F, d) = kFxNoExp;
+    }
+    if (a.ubar_old && live) a.ubar_old[(size_t)element(el) * Q + q] = ud[k.col];
+  }
+  fx_sync<S::NT>();
+  if (k.act)
+    for (int b = k.line; b < NP_S; b += S::LINES)
+      k.m[S::O_U + b * LD + k.col] = fx_from_double(ud[b * LD + k.col], k.word(S::I_EU));
   fx_sync<S::NT>();
 }
 
@@ -760,27 +797,7 @@ __device__ __forceinline__ void fx_predictor_chunk(const PredictorArgs& a, char*
   fx_load_coefs<O>(D == 2 ? k.line % N : (k.line / N) % N, c1);
   if constexpr (D == 3) fx_load_coefs<O>(k.line % N, c2);
 
-  // U: coalesced loads, the column's exponent, fixed point
-  double* ud = reinterpret_cast<double*>(k.m + S::O_G);
-  for (int i = threadIdx.x; i < C * NP_S; i += NT)
-    ud[(i % NP_S) * LD + i / NP_S] = a.Uw[(size_t)element(i / (Q * NP_S)) * Q * NP_S + i % (Q * NP_S)];
-  fx_sync<S::NT>();
-  if (k.act && k.line == 0) {
-    const int eu = fx_norm_exp<NP_S>(ud + k.col, LD);
-    k.word(S::I_EU) = eu;
-    k.word(S::I_SUM) = k.word(S::I_N) = k.word(S::I_F64) = 0;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      k.word(S::I_Z, d) = 0;
-      k.word(S::I_F, d) = kFxNoExp;
-    }
-    if (a.ubar_old && live) a.ubar_old[(size_t)e * Q + q] = ud[k.col];
-  }
-  fx_sync<S::NT>();
-  if (k.act)
-    for (int b = k.line; b < NP_S; b += S::LINES)
-      k.m[S::O_U + b * LD + k.col] = fx_from_double(ud[b * LD + k.col], k.word(S::I_EU));
-  fx_sync<S::NT>();
+  fx_load_state<O, E>(k, a, element, live);
 
   // the first sweep on U, then the others (AmrDG.h:1103-1119)
   {
@@ -829,8 +846,9 @@ __device__ __forceinline__ void fx_predictor_chunk(const PredictorArgs& a, char*
       fx_line_points<O>(t, [&](int k0, long long v) { h[k0 * S::LINES * LD] = fx_to_double(v, eh, nan_bits); });
       if (live) {
         double* tr = a.Tr + (size_t)e * NF * TT + q * NB + kt * NSB;
-        fx_face_values<O, E>(k, t, eh, nan_bits, tr);
-        fx_side_lines<O, E>(k, g, eh, nan_bits, tr);
+        auto out = [&](int face, int x, long long v) { tr[face * TT + x] = fx_to_double(v, eh, nan_bits); };
+        fx_face_values<O, E>(k, t, out);
+        fx_side_lines<O, E>(k, g, out);
       }
     }
     fx_sync<S::NT>();
@@ -862,7 +880,7 @@ __device__ __forceinline__ void fx_predictor_chunk(const PredictorArgs& a, char*
     }
   }
   fx_sync<S::NT>();
-  fx_volume_term<O, E>(k);
+  fx_volume_term<O, E, false>(k);
   // Rvol = M U + sum_d (Dt/dx_d) Sk_d F_d, coalesced
   const double* vt = reinterpret_cast<const double*>(k.m + S::O_A);
   for (int i = threadIdx.x; i < C * NP_S; i += NT) {
@@ -894,6 +912,133 @@ template <class O, int E>
 __global__ void __launch_bounds__((FxShape<O, E>::NT), (FxShape<O, E>::MIN_BLOCKS)) k_predictor_fx(PredictorArgs a) {
   extern __shared__ __align__(16) char fx_smem[];
   fx_predictor_chunk<O, E>(a, fx_smem, blockIdx.x, a.n_elem);
+}
+
+// The time-independent part of a seeded step's final stage (split_epilogue of
+// adg_kernels.cuh): the volume term of F(U) to Rvol, and U and its normal
+// flux at the faces' spatial points to the split trace tiles.  In the FP64 of
+// the seeded kernel this was 1850 of its 2050 FP64 operations an element and
+// kept that pipe 65 % busy; one slice of the plain predictor's stages does it
+// on the integer pipes.  D2P3, 15,600 elements: 27 us (blocks of 16 elements
+// 30), the seeded kernel 45 us, where it was 90 us with both.
+template <class O, int E>
+struct FxBase {
+  using S = FxShape<O, E>;
+  static constexpr int NSB = O::NQ_BD / O::N, NF = 2 * O::D;
+  // the face values lie in the accumulators' place and behind it
+  static constexpr int SLOTS = S::O_A + NF * NSB * S::LD > S::SLOTS ? S::O_A + NF * NSB * S::LD : S::SLOTS;
+  static constexpr size_t BYTES = (size_t)SLOTS * 8 + (size_t)S::WORDS * 4;
+};
+
+template <class O, int E>
+__global__ void __launch_bounds__((FxShape<O, E>::NT), (FxShape<O, E>::MIN_BLOCKS)) k_split_base(PredictorArgs a) {
+  using S = FxShape<O, E>;
+  constexpr int D = O::D, Q = O::Q, N = O::N, NP_S = O::NP_S, LD = S::LD, C = S::C, NT = S::NT;
+  constexpr int NSB = FxBase<O, E>::NSB, NF = 2 * D, TT = tr_tile<O>();
+  extern __shared__ __align__(16) char fx_smem[];
+  FxBlock<O, E> k;
+  k.m = reinterpret_cast<long long*>(fx_smem);
+  k.w = reinterpret_cast<int*>(k.m + FxBase<O, E>::SLOTS);
+  k.line = threadIdx.x / S::CP;
+  k.act = k.line < S::LINES && (int)threadIdx.x % S::CP < C;
+  k.col = k.act ? threadIdx.x % S::CP : 0;
+  const int e0 = blockIdx.x * E, limit = a.n_elem;
+  auto element = [&](int el) {  // past the end: the last one (its results are not written)
+    const int i = e0 + el < limit ? e0 + el : limit - 1;
+    return a.elem_list ? a.elem_list[i] : i;
+  };
+  const double gm1 = a.gamma - 1.0;
+  const FxFactor gm1x = fx_factor(gm1);
+  FxCoef c1[N], c2[N];
+  fx_load_coefs<O>(D == 2 ? k.line % N : (k.line / N) % N, c1);
+  if constexpr (D == 3) fx_load_coefs<O>(k.line % N, c2);
+  fx_load_state<O, E>(k, a, element, e0 + k.col / Q < limit);
+  // U at the points and the faces' points
+  const long long* g = k.m + S::O_U;
+  long long* faces = k.m + S::O_A;
+  if (k.act) {
+    long long t[N];
+    fx_line_modes<O, LD>(g + k.col, c1, c2, t);
+    long long* h = k.m + S::O_F + k.line * LD + k.col;
+    int n = 0;
+    fx_line_points<O>(t, [&](int k0, long long v) {
+      h[k0 * S::LINES * LD] = v;
+      n = max(n, __clz((int)(v >> 32)));
+    });
+    auto out = [&](int face, int x, long long v) {
+      faces[(face * NSB + x) * LD + k.col] = v;
+      n = max(n, __clz((int)(v >> 32)));
+    };
+    fx_face_values<O, E>(k, t, out);
+    fx_side_lines<O, E>(k, g, out);
+    if (k.col % Q == 0) atomicMax(&k.word(S::I_N), n);
+  }
+  fx_sync<NT>();
+  fx_point_fluxes<O, E, true>(k, true, gm1, gm1x);
+  // the faces' spatial points: U and the normal flux
+  const int* wx = k.w + S::I_EU;
+#pragma unroll 1
+  for (int it = threadIdx.x; it < E * NF * NSB; it += NT) {
+    const int p = it % (NF * NSB), c0 = it / (NF * NSB) * Q, dir = p / (2 * NSB);
+    if (e0 + c0 / Q >= limit) break;
+    double* tile = a.Tr + ((size_t)element(c0 / Q) * NF + p / NSB) * TT + p % NSB;
+    long long u[Q];
+#pragma unroll
+    for (int v = 0; v < Q; ++v) {
+      u[v] = faces[p * LD + c0 + v];
+      tile[v * NSB] = fx_to_double(u[v], wx[c0 + v], fx_poison(wx[c0 + v]));
+    }
+    int em[D], range = max(abs(wx[c0] - 1022), abs(wx[c0 + D + 1] - 1022));
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      em[d] = wx[c0 + d + 1];
+      range = max(range, em[d] - 1022);
+    }
+    const int n = k.w[S::I_N + c0];
+    const FxFluxExp<D> x(em, wx[c0 + D + 1], wx[c0], n, gm1x.ef);
+    long long F[D][D + 1];
+    double* f = tile + Q * NSB;
+    if (range < 480 && fx_euler_flux<D>(u, x, wx[c0 + D + 1], n, gm1x, F)) {
+#pragma unroll
+      for (int v = 0; v < Q; ++v) {
+        long long y = 0;
+        int e = 0;
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+          if (d == dir) {
+            y = v ? F[d][v > 0 ? v - 1 : 0] : u[d + 1];
+            e = v ? x.flux(d, v, em) : em[d];
+          }
+        f[v * NSB] = fx_to_double(y, e, 0);
+      }
+    } else {
+      double uu[Q], F64[Q];
+#pragma unroll
+      for (int v = 0; v < Q; ++v) uu[v] = fx_to_double(u[v], wx[c0 + v], fx_poison(wx[c0 + v]));
+      (void)euler_flux_normal<D>(dir, uu, a.gamma, F64);
+#pragma unroll
+      for (int v = 0; v < Q; ++v) f[v * NSB] = F64[v];
+    }
+  }
+  fx_sync<NT>();
+  fx_volume_term<O, E, true>(k);
+  // Rvol = M U + sum_d (Dt/dx_d) (sum_k w_k) Sk_d F_d(U), coalesced
+  double* cw = reinterpret_cast<double*>(k.m + S::O_H);  // [element][d]
+  for (int i = threadIdx.x; i < E * D; i += NT) {
+    const int lev = a.elem_level ? a.elem_level[element(i / D)] : 0;
+    cw[i] = a.dt[kScalDtDx + 3 * lev + i % D] * O::WEIGHT_SUM;
+  }
+  fx_sync<NT>();
+  const double* vt = reinterpret_cast<const double*>(k.m + S::O_A);
+  for (int i = threadIdx.x; i < C * NP_S; i += NT) {
+    const int b = i % NP_S, cc = i / NP_S;
+    if (e0 + cc / Q >= limit) continue;
+    const size_t o = (size_t)element(cc / Q) * Q * NP_S + i % (Q * NP_S);
+    double r = O::mdiag(b) * a.Uw[o];
+#pragma unroll
+    for (int d = 0; d < D; ++d) r = fma(cw[cc / Q * D + d], vt[(d * NP_S + b) * LD + cc], r);
+    a.Rvol[o] = r;
+  }
 }
 
 // The fallback pass: a short grid striding over a list counted on the device.
