@@ -464,6 +464,7 @@ int upload_tables(adg_ctx* ctx, const RemapTable* rm = nullptr) {
 
 }  // namespace
 int launch_seeded_predictor(adg_ctx* ctx, const PredictorArgs& base, cudaEvent_t* ev);
+int seeded_elems(const adg_ctx* ctx);
 namespace {
 
 int flush_ghosts(adg_ctx* ctx);
@@ -2348,7 +2349,7 @@ int adg_block_choices(const adg_ctx* ctx, int* choices, int cap, int* n, int* E_
   for (int i = 0; i < cap && choices && i < (int)ch.size(); ++i) choices[i] = ch[i];
   if (n) *n = (int)ch.size();
   if (E_plain) *E_plain = ctx->E;
-  if (E_seeded) *E_seeded = ctx->Es > 0 ? ctx->Es : (ctx->seed_mode == 2 && ctx->cfg.D == 2 ? 8 : ctx->E);
+  if (E_seeded) *E_seeded = seeded_elems(ctx);
   return ADG_OK;
 }
 
@@ -2697,16 +2698,49 @@ int seed_infer(adg_ctx* ctx, double* dst, int path, float* dst_f = nullptr) {
   return ADG_OK;
 }
 
+// Elements per block of the FP64 column kernels (mode 1, and mode 3's fallback
+// lists) where neither the caller nor the autotuner chose: not the plain
+// path's (a seeded step of 100^2 D2P3 with many elements falling back, 8 / 16:
+// 775 / 547 us).
+int column_elems(const adg_ctx* ctx) {
+  const std::vector<int> ch = ctx->ks->elems_per_block_choices();
+  const int E = ctx->E_default ? (ctx->cfg.D == 2 ? 16 : 8) : ctx->E;
+  return std::find(ch.begin(), ch.end(), E) != ch.end() ? E : ctx->E;
+}
+// and of the seeded predictor
+int seeded_elems(const adg_ctx* ctx) {
+  return ctx->Es > 0 ? ctx->Es : ctx->seed_mode == 2 && ctx->cfg.D == 2 ? 8 : column_elems(ctx);
+}
+
 int launch_seeded_predictor(adg_ctx* ctx, const PredictorArgs& base, cudaEvent_t* ev) {
   const int n = (int)ctx->hier.n_elem();
   const KernelSet* ks = ctx->ks;
   cudaStream_t st = ctx->stream;
   // FP32 sweeps from the tensor-core path take an FP32 seed
   const bool f32 = ctx->seed_mode == 2 && ctx->seed_path == 1 && ctx->seed->packed;
+  // the time-independent part needs no seed: on the side stream beside the
+  // inference where that (128 elements a block) leaves half of the SMs idle
+  // (48^2 D2P2 97 -> 93 us a step, D2P3 209 -> 203; 15,600 elements 242 ->
+  // 246: not there, and not while stages are timed)
+  const bool split = ctx->seed_mode == 2 && ks->split_base_apart();
+  const bool fork = split && !ev && ctx->side && n <= 76 * 128;
+  if (fork) {
+    ADG_CUDA(cudaEventRecord(ctx->fork_ev, st), "fork");
+    ADG_CUDA(cudaStreamWaitEvent(ctx->side, ctx->fork_ev, 0), "fork");
+  }
   int rc = seed_infer(ctx, ctx->hseed.p, ctx->seed_path, f32 ? ctx->hseed_f.p : nullptr);
+  cudaError_t e = cudaSuccess;
+  if (rc == ADG_OK && ev) cudaEventRecord(ev[6], st);  // end of the seed inference (stage timing)
+  if (split) {
+    e = ks->split_base(base, fork ? ctx->side : st);
+    ctx->launches++;
+    if (fork) {  // joined whatever failed
+      ADG_CUDA(cudaEventRecord(ctx->join_ev, ctx->side), "join");
+      ADG_CUDA(cudaStreamWaitEvent(st, ctx->join_ev, 0), "join");
+    }
+  }
   if (rc) return rc;
-  if (ev) cudaEventRecord(ev[6], st);  // end of the seed inference (stage timing)
-  cudaError_t e;
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "time-independent part");
   ADG_CUDA(cudaMemsetAsync(ctx->fb_count.p, 0, sizeof(int), st), "fallback reset");
   PredictorArgs pa = base;
   pa.Hseed = ctx->hseed.p;
@@ -2718,13 +2752,7 @@ int launch_seeded_predictor(adg_ctx* ctx, const PredictorArgs& base, cudaEvent_t
   // the FP32 predictor at D = 2 runs one-warp blocks (8 elements): 16 of them
   // per SM, so the element groups spread evenly over the SMs (at D = 3 the
   // 40-thread blocks of 8 elements idle 3/8 of their lanes: the tuned E stays)
-  const int Es = ctx->Es > 0 ? ctx->Es : (ctx->seed_mode == 2 && ctx->cfg.D == 2 ? 8 : ctx->E);
-  if (ctx->seed_mode == 2) {
-    e = ks->split_base(pa, st);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "time-independent part");
-    ctx->launches++;
-  }
-  e = ks->predictor(pa, Es, st, ctx->seed_mode);
+  e = ks->predictor(pa, seeded_elems(ctx), st, ctx->seed_mode);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "seeded predictor");
   if (ev) cudaEventRecord(ev[7], st);  // end of the seeded predictor, start of the fallback pass
   // full FP64 Picard for the rejected elements; in a mode-2 step with the
@@ -2733,7 +2761,7 @@ int launch_seeded_predictor(adg_ctx* ctx, const PredictorArgs& base, cudaEvent_t
   fb.elem_list = ctx->fb_list.p;
   fb.list_count = ctx->fb_count.p;
   fb.count_total = ctx->fb_total.p;
-  e = ks->predictor(fb, ctx->E, st, ctx->seed_mode == 2 ? 3 : 0);
+  e = ctx->seed_mode == 2 ? ks->predictor(fb, column_elems(ctx), st, 3) : ks->predictor(fb, ctx->E, st, 0);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "fallback predictor");
   ctx->launches += 2;
   return ADG_OK;

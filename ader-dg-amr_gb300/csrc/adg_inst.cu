@@ -23,7 +23,7 @@ constexpr size_t smem_bytes() {
   constexpr size_t ld = E * O::Q + 1;
   constexpr bool split = MODE == 2 || MODE == 3;
   constexpr size_t sweeps = MODE == 2 ? O::D * O::NQ_S * ld * sizeof(float) : O::D * O::NQ_ST * ld * sizeof(double);
-  constexpr size_t fin = split ? split_epilogue_doubles<O>(ld, MODE == 3) * sizeof(double)
+  constexpr size_t fin = split ? split_epilogue_doubles<O>(ld, MODE == 3 || !base_apart<O>()) * sizeof(double)
                                : (1 + O::D) * O::NQ_S * ld * sizeof(double);
   constexpr size_t faces = split ? 0 : 2 * O::NQ_BD * ld * sizeof(double);
   constexpr size_t red = 2 * E * O::Q * sizeof(double);
@@ -182,11 +182,10 @@ struct Impl final : KernelSet {
   }
 #endif
   cudaError_t split_base(const PredictorArgs& a, cudaStream_t s) const override {
-    if constexpr (kSeedModes) {
-      return launch_split_base<O::D == 2 ? 8 : 6>(a, s);
-    }
+    if constexpr (kSeedModes && base_apart<O>()) return launch_split_base<O::D == 2 ? 8 : 6>(a, s);
     return cudaErrorNotSupported;
   }
+  bool split_base_apart() const override { return kSeedModes && base_apart<O>(); }
   cudaError_t numflux(const FaceArgs& a, long long nface, cudaStream_t s, bool split) const override {
     if (nface <= 0) return cudaSuccess;
     constexpr int FB = numflux_faces_per_block<O>();

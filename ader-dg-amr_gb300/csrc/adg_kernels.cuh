@@ -313,6 +313,14 @@ __device__ __forceinline__ void face_traces(const double* hw, double* sm, int co
 // there already, in Rvol and the tiles (k_split_base of adg_predictor_fx.cuh).
 // ---------------------------------------------------------------------------
 
+// D2P1 does both in one kernel: its FP64 work is less than a launch (100^2 /
+// 256^2 elements: 14.5 / 69 us in one, 17.4 / 63 in two).
+template <class O>
+constexpr bool base_apart() {
+  return O::D == 3 || O::P > 1;
+}
+
+
 // Shared memory of split_epilogue (doubles).  BASE: D NS ld doubles (U, then
 // F(U) at the spatial points; later the FP32 delta slice and flux change
 // sums), then NS ld floats of U in FP32; else D + 1 such slabs of floats and
@@ -749,7 +757,7 @@ __device__ __forceinline__ void predictor_chunk(const PredictorArgs& a, double* 
 #pragma unroll
       for (int n = 0; n < NP_S; ++n) uf[n] = (float)u[n];
     }
-    split_epilogue<O, E, MODE == 3>(u, uf, dlt, c, gm1, sm, col, q, live, e, e0, limit, a);
+    split_epilogue<O, E, MODE == 3 || !base_apart<O>()>(u, uf, dlt, c, gm1, sm, col, q, live, e, e0, limit, a);
   } else {
     fp64_epilogue<O, E>(hw, u, c, gm1, sm, col, q, live, e, e0, limit, a);
   }

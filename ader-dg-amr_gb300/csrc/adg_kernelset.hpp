@@ -32,6 +32,7 @@ struct KernelSet {
   // the time-independent part of mode 2's final stage, before that mode's
   // launch on the same elements
   virtual cudaError_t split_base(const PredictorArgs& a, cudaStream_t s) const = 0;
+  virtual bool split_base_apart() const = 0;  // else mode 2 does it itself
   // split: the trace tiles are split tiles (predictor modes 2 and 3);
   // nface: the faces computed (a.n_list with a face list)
   virtual cudaError_t numflux(const FaceArgs& a, long long nface, cudaStream_t s, bool split = false) const = 0;
