@@ -356,21 +356,21 @@ def l2_density_level0(Ua, Ub, w):
 L2_FLUSH_BYTES = 256 << 20  # twice the 129 MB L2: written before every timed step
 
 # Per launch of the dominant kernels on the headline workload (ncu, same
-# code and layout; profiles/fp64_issue_k_predictor_kh_p3_amr3.md): FP64-pipe
-# thread instruction slots (smsp__inst_executed_pipe_fp64 x 32), the
-# DFMA+DADD+DMUL part of them, DRAM bytes read + written, FP64 pipe activity,
-# elements predicted.
+# code and layout; profiles/fp64_issue_k_predictor_kh_p3_amr3.md): warp
+# instructions issued, FP64-pipe thread instruction slots
+# (smsp__inst_executed_pipe_fp64 x 32), the DFMA+DADD+DMUL part of them, DRAM
+# bytes read + written, issue and FP64 pipe activity, elements predicted.
 PROFILED_LAUNCH = {
     "kh_p3_amr3": {
-        "plain_predictor": dict(kernel="k_predictor<D2P3, E=8, MODE 0> (3 FP64 Picard sweeps, corrector volume "
+        "plain_predictor": dict(kernel="k_predictor_fx<D2P3, E=8> (3 Picard sweeps in fixed point, corrector volume "
                                        "term, face traces)",
-                                fp64_pipe_slots=301.576e6, fp64_arith=296.329e6, dram_bytes=24.63e6,
-                                fp64_active=0.756, elements=15616,
+                                inst=165.907e6, fp64_pipe_slots=52.345e6, fp64_arith=49.347e6, dram_bytes=29.95e6,
+                                issue_active=0.485, fp64_active=0.305, elements=15616,
                                 source="profiles/fp64_issue_k_predictor_kh_p3_amr3.md"),
-        "seeded_predictor": dict(kernel="k_predictor<D2P3, E=8, MODE 2> (2 FP32 sweeps from the seed, split "
-                                        "FP64/FP32 final stage)",
-                                 fp64_pipe_slots=34.855e6, fp64_arith=29.436e6, dram_bytes=16.89e6,
-                                 fp64_active=0.633, elements=15616,
+        "seeded_predictor": dict(kernel="k_split_base<D2P3, E=8> (time-independent part in fixed point) and "
+                                        "k_predictor<D2P3, E=8, MODE 2> (2 FP32 sweeps from the seed, FP32 changes)",
+                                 inst=37.752e6, fp64_pipe_slots=5.309e6, fp64_arith=3.670e6, dram_bytes=29.52e6,
+                                 issue_active=0.442, fp64_active=0.122, elements=15616,
                                  source="profiles/fp64_issue_k_predictor_kh_p3_amr3.md"),
     },
 }
@@ -588,10 +588,11 @@ def e2e_device_patches(G, s, w, steps):
 
 
 def roofline_line(G, w, workload, head_name, km_head, km_plain, el_per_step):
-    """roofline of the headline path's dominant kernel: FP64-pipe issue (the
-    ncu-counted FP64-pipe instruction slots of one launch, 2 flops each as the
-    DFMA peak counts them) over the live CUDA-event duration, against the DFMA
-    issue rate measured in this run."""
+    """roofline of the headline path's dominant kernels: instruction issue (the
+    ncu-counted warp instructions of one launch over the live CUDA-event
+    duration, against four a clock and SM at 2070 MHz), and beside it the FP64
+    pipe's (its instruction slots, 2 flops each, against the DFMA rate measured
+    in this run)."""
     from math import comb
 
     D, P = w["D"], w["P"]
@@ -604,29 +605,34 @@ def roofline_line(G, w, workload, head_name, km_head, km_plain, el_per_step):
     key = "seeded_predictor" if seeded else "plain_predictor"
     t = km_head["seeded_predictor"] if seeded else km_plain["predictor"]
     prof = PROFILED_LAUNCH.get(workload, {}).get(key)
-    line = {"bound": "fp64", "unit": "TFLOP/s", "peak": peak,
-            "peak_source": "FP64 DFMA-chain probe on this GPU in this run (adg_fp64_peak_probe; "
-                           "MEASURED_PEAKS.json has no FP64 figure)",
+    issue_peak = 4 * 152 * 2.07  # warp instructions per ns
+    line = {"bound": "issue", "unit": "G warp instructions/s", "peak": issue_peak,
+            "peak_source": "four schedulers on each of 152 SMs at the 2070 MHz of the sampled clocks",
+            "fp64_peak_tflops": peak,
+            "fp64_peak_source": "FP64 DFMA-chain probe on this GPU in this run (adg_fp64_peak_probe; "
+                                "MEASURED_PEAKS.json has no FP64 figure)",
             "kernel_ms": t}
     if prof:
-        achieved = 2.0 * prof["fp64_pipe_slots"] / (t * 1e-3) / 1e12
+        achieved = prof["inst"] / (t * 1e-3) / 1e9
         line.update({
-            "kernel": prof["kernel"], "achieved": achieved, "frac": achieved / peak,
+            "kernel": prof["kernel"], "achieved": achieved, "frac": achieved / issue_peak,
+            "issue_active_ncu": prof["issue_active"],
+            "fp64_issue_frac": 2.0 * prof["fp64_pipe_slots"] / (t * 1e-3) / 1e12 / peak,
             "traffic": prof["dram_bytes"], "traffic_source": prof["source"],
             "fp64_pipe_slots_per_launch": prof["fp64_pipe_slots"],
             "fp64_arith_frac": 2.0 * prof["fp64_arith"] / (t * 1e-3) / 1e12 / peak,
             "fp64_pipe_active_ncu": prof["fp64_active"],
             "elements_per_launch": prof["elements"],
             "effective_dense_tflops": alg_pred * prof["elements"] / (t * 1e-3) / 1e12,
-            "note": ("achieved = the kernel's FP64-pipe instruction slots per launch (ncu) x 2 / its event-timed "
-                     "duration: the FP64 issue rate, cross-checked by fp64_pipe_active_ncu; "
+            "note": ("achieved = the kernels' warp instructions per launch (ncu) / their event-timed duration, "
+                     "cross-checked by issue_active_ncu; "
                      "effective_dense_tflops counts the method's dense matrix-form flops per element (" +
                      f"{alg_pred:.0f}) instead, which the generated sum-factorised operators do not issue"),
         })
     else:
         line.update({"kernel": key, "achieved": None, "frac": None, "traffic": None,
                      "effective_dense_tflops": alg_pred * el_per_step / (t * 1e-3) / 1e12,
-                     "note": "no FP64 instruction count profiled for this workload"})
+                     "note": "no instruction count profiled for this workload"})
     return line
 
 
@@ -857,7 +863,7 @@ def run_ours(args, w):
         # the seed network runs over every element of the layout, the
         # coarse-fine ghosts included: its count over the same three steps
         seed_el = (G.seed_stats(head["sim"])[1] - n_seed0) / 3.0
-        roof["seed_path"] = seed_roofline(w, km_head, seed_el, roof["peak"])
+        roof["seed_path"] = seed_roofline(w, km_head, seed_el, roof["fp64_peak_tflops"])
     line = {
         "metric": METRIC, "value": value, "unit": "DOF-updates/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
