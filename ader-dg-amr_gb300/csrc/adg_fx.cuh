@@ -144,15 +144,22 @@ __device__ __forceinline__ long long fx_mul(int ah, int al, int bh, int bl) {
   return s.get();
 }
 
+__device__ __forceinline__ float fx_rcp_estimate(float x) {
+#ifdef __CUDACC__
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else  // a host build (tests)
+  return 1.0f / x;
+#endif
+}
+
 // Reciprocal of v, 2^40 <= v < 2^60, n = clz(v): 2^(123 - n) / v, in
 // (2^59, 2^60].  The FP32 estimate r of the significand x in [1, 2) (24
 // bits), e = 1 - x r exactly, one third-order Householder step r (1 + e + e^2).
 __device__ __forceinline__ long long fx_reciprocal(long long v, int n) {
   const unsigned long long x = (unsigned long long)v << (n - 4);  // [2^59, 2^60)
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;"
-      : "=f"(r)
-      : "f"(__int_as_float(0x3f800000 | (((int)(x >> 36)) & 0x7fffff))));
+  const float r = fx_rcp_estimate(__int_as_float(0x3f800000 | (((int)(x >> 36)) & 0x7fffff)));
   const unsigned r0 = (unsigned)__float2int_rn(r * 16777216.0f);  // 2^24 r, exact
   const long long e = -(long long)(x * r0);                       // 2^83 e: the product's 2^83 leaves 64 bits
   const int eh = (int)(e >> 32);
@@ -186,6 +193,14 @@ __device__ __forceinline__ int fx_norm_exp(const double* x, int s) {
 // intermediate values are the element's, so a point does no normalisation
 // but the density's.
 // ---------------------------------------------------------------------------
+
+// Smallest pressure the integer path takes, as a column value of exponent x:
+// the model's floor, 10 2^-52 = 5 2^(1031 - 1082), which the FP64 evaluation
+// applies, and 2^-40 of the bound.
+__device__ __forceinline__ long long fx_min_pressure(int x) {
+  const int s = 1031 - x;
+  return s < 18 ? 1LL << 20 : 5LL << (s < 60 ? s : 60);
+}
 
 // Exponents: em momenta, ee energy, er density; n: the largest number of
 // leading zeros of the element's densities, which bounds 1 / rho; gef: that
@@ -235,8 +250,8 @@ constexpr long long kFxMinRho = 1LL << 40;
 constexpr int kFxRhoSpan = 6;
 
 // Fluxes F[d][q - 1], q >= 1, at exponents x.flux(d, q).  False where the
-// density is out of range or the pressure within 2^-40 of its terms (or at
-// the floor): such points are for the FP64 evaluation.
+// density is out of range or the pressure below fx_min_pressure: such points
+// are for the FP64 evaluation.
 template <int D>
 __device__ __forceinline__ bool fx_euler_flux(const long long* u, const FxFluxExp<D>& x, int ee, int n_max,
                                               const FxFactor& gm1, long long (&F)[D][D + 1]) {
@@ -263,7 +278,7 @@ __device__ __forceinline__ bool fx_euler_flux(const long long* u, const FxFluxEx
     p -= fx_align(w[d], top - x.xk[d] + 1);
   }
   p = fx_scale(p, gm1);
-  if (p < (1LL << 20)) return false;
+  if (p < fx_min_pressure(x.xp)) return false;
   const long long ep = fx_align(u[D + 1], x.xe - ee) + fx_align(p, x.xe - x.xp);
   const int eh = fx_hi(ep), el = fx_lo(ep);
 #pragma unroll
