@@ -19,8 +19,9 @@
 //
 // Phase 3 evaluates the fluxes on the column values (fx_euler_flux); an
 // element with a point whose density or pressure is out of that form's range
-// (near vacuum, at the pressure floor, densities more than 2^6 apart) takes
-// the FP64 fluxes for all of its points, and so do values that are not finite.
+// (near vacuum, at the pressure floor, densities more than 2^2 apart, kinetic
+// terms whose bound is more than 2^4 above the energy's) takes the FP64 fluxes
+// for all of its points, and so do values that are not finite.
 //
 // Why this form: GB300 issues 1.6 FP64 operations per clock and SM.  The
 // column-per-thread FP64 predictor kept that pipe 84 % busy; with the
