@@ -68,14 +68,14 @@ __device__ __forceinline__ int fx_poison(int E) { return E > kFxMaxExp ? 0x7ff80
 
 // x as a column value of exponent E >= the exponent field of x (exact down to
 // 2^-7 of the bound, truncated toward zero below; a negative x one unit
-// lower: its complement, not its negative).
+// lower: its complement, not its negative); zero and subnormal numbers zero.
 __device__ __forceinline__ long long fx_from_double(double x, int E) {
   const int hi = __double2hiint(x), lo = __double2loint(x);
   const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
   const unsigned long long m = ((unsigned long long)mh << 39) | ((unsigned long long)(unsigned)lo << 7);
-  const int r = E - ((hi >> 20) & 0x7ff);
+  const int f = (hi >> 20) & 0x7ff, r = E - f;
   const long long s = hi >> 31;  // 0 or -1
-  return (long long)(m >> (r < 63 ? r : 63)) ^ s;
+  return f ? (long long)(m >> (r < 63 ? r : 63)) ^ s : 0;
 }
 
 // Column value to the nearest double (a negative one from its complement);
@@ -99,8 +99,8 @@ static __device__ __noinline__ double fx_to_double_small(long long v, int E, int
   const int n = __clzll((long long)a);
   const unsigned long long m = n < 64 ? a << n : 0;
   const int ef = E + 3 - n;
-  unsigned long long d = (m >> 11) + ((m >> 10) & 1) + ((unsigned long long)(unsigned)ef << 52);
-  if (ef < 0 || (long long)m >= 0) d = 0;
+  const unsigned long long d = (m >> 11) + ((m >> 10) & 1) + ((unsigned long long)(unsigned)ef << 52);
+  if (ef < 0 || (long long)m >= 0) return __hiloint2double(nan_bits, 0);
   return __hiloint2double((int)(d >> 32) | ((int)s & (int)0x80000000) | nan_bits, (int)d);
 }
 

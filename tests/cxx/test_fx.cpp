@@ -64,6 +64,34 @@ static void pressure_floor() {
       }
 }
 
+// A column of zeros or subnormal numbers is zero, whatever its exponent and
+// however its values are added up, and so is a zero in any column; a value is
+// the double itself while its bits are above 2^-60 of the bound.
+static void zero_columns() {
+  for (double z : {0.0, -0.0, 4.9e-324, -2.2e-308}) {
+    const double x[10] = {z, -z, z, z, z, z, -z, z, z, z};
+    for (int E : {fx_norm_exp<10>(x, 1), 1, 60, 64, 1022, 2039}) {
+      long long sum = 0;
+      for (double y : x) {
+        CHECK(fx_from_double(y, E) == 0, "%g in a column of exponent %d is %lld", y, E, fx_from_double(y, E));
+        sum += fx_from_double(y, E);
+      }
+      const double back = fx_to_double(sum, E, 0);
+      CHECK(back == 0.0 && !std::signbit(back), "the sum of a column of %g is %g", z, back);
+      CHECK(fx_to_double(-1, 3, 0) == 0.0 && !std::signbit(fx_to_double(-1, 3, 0)), "-1 unit below the doubles");
+    }
+  }
+  std::mt19937_64 rng(1);
+  for (int i = 0; i < 1000000; ++i) {
+    const int e = 8 + (int)(rng() % 2030);
+    const double x = __longlong_as_double((long long)((rng() & 0x800fffffffffffffULL) | (unsigned long long)e << 52));
+    for (int up = 0; up < 8 && e + up <= kFxMaxExp; ++up) {
+      const double back = fx_to_double(fx_from_double(x, e + up), e + up, 0);
+      CHECK(back == x, "%a in a column of exponent %d is %a", x, e + up, back);
+    }
+  }
+}
+
 // 113-bit arithmetic: the measure of both forms of the fluxes.
 #ifdef __SIZEOF_FLOAT128__
 typedef __float128 wide;
@@ -241,6 +269,8 @@ int main(int argc, char** argv) {
   if (what == "pressure_floor") {
     pressure_floor<2>();
     pressure_floor<3>();
+  } else if (what == "zero_columns") {
+    zero_columns();
   } else if (what == "flux_accuracy") {
     flux_accuracy();
   } else {

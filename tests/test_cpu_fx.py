@@ -22,7 +22,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("check", ["pressure_floor", "flux_accuracy"])
+@pytest.mark.parametrize("check", ["pressure_floor", "flux_accuracy", "zero_columns"])
 def test_fixed_point_columns(exe, check):
     r = subprocess.run([exe, check], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
