@@ -17,6 +17,7 @@
 #include "adg_kernelset.hpp"
 #include "adg_layout.hpp"
 #include "adg_mlp.cuh"
+#include "adg_orders.hpp"
 #include "adg_patches.cuh"
 #include "plotfile.hpp"
 #include <random>
@@ -86,6 +87,52 @@ __global__ void k_fp64_probe(double* out, int iters) {
 
 using namespace adg;
 
+// send_order's buffers, page-locked, and theirs on the device, kept with the
+// seed.  The copies run on a stream of their own beside the epoch before (in
+// the training stream a copy's latency showed: 4 us an epoch of 266).
+struct OrderPort {
+  int *host = nullptr, *dev = nullptr;
+  size_t cap = 0;  // of one buffer
+  cudaEvent_t copied[2] = {}, used[2] = {};
+  cudaStream_t side = nullptr, train = nullptr;
+  cudaError_t ensure(size_t n) {
+    cudaError_t rc = cudaSuccess;
+    for (auto* e : {copied, used})
+      for (int b = 0; b < 2 && rc == cudaSuccess; ++b)
+        if (!e[b]) rc = cudaEventCreateWithFlags(&e[b], cudaEventDisableTiming);
+    if (rc == cudaSuccess && !side) rc = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+    if (rc != cudaSuccess || n <= cap) return rc;
+    free_buffers();  // (idle: training waits for its own work)
+    rc = cudaMallocHost(&host, 2 * n * sizeof(int));
+    if (rc == cudaSuccess) rc = cudaMalloc(&dev, 2 * n * sizeof(int));
+    if (rc == cudaSuccess) cap = n;
+    return rc;
+  }
+  bool wait(int b) { return cudaEventSynchronize(copied[b]) == cudaSuccess; }
+  int* buffer(int b, size_t) { return host + b * cap; }
+  const int* order(int b) const { return dev + b * cap; }
+  bool copy(int b, size_t n) {
+    return cudaStreamWaitEvent(side, used[b], 0) == cudaSuccess &&
+           cudaMemcpyAsync(dev + b * cap, host + b * cap, n * sizeof(int), cudaMemcpyHostToDevice, side) ==
+               cudaSuccess &&
+           cudaEventRecord(copied[b], side) == cudaSuccess && cudaStreamWaitEvent(train, copied[b], 0) == cudaSuccess;
+  }
+  bool done(int b) { return cudaEventRecord(used[b], train) == cudaSuccess; }  // the order has been read
+  void free_buffers() {
+    if (host) cudaFreeHost(host);
+    if (dev) cudaFree(dev);
+    host = dev = nullptr;
+    cap = 0;
+  }
+  void release() {
+    free_buffers();
+    for (auto* e : {copied, used})
+      for (int b = 0; b < 2; ++b)
+        if (e[b]) cudaEventDestroy(e[b]);
+    if (side) cudaStreamDestroy(side);
+  }
+};
+
 struct adg_seed {
   int D = 2, P = 1, Q = 4, n_in = 0, n_out = 0, h = 128;
   const KernelSet* ks = nullptr;
@@ -100,7 +147,7 @@ struct adg_seed {
   DevBuf<float> Z1, A1, Z2, A2, Z3, A3, dY, dA, dZ, Xb, Tb;
   DevBuf<float> red;  // slices of the weight gradients (added in order)
   long long work_rows = 0;
-  DevBuf<int> idx;
+  OrderPort orders;
   DevBuf<double> loss;
   std::mt19937_64 rng;
   long long adam_t = 0;
@@ -113,7 +160,7 @@ struct adg_seed {
     DevBuf<float>* bufs[] = {&params, &grads, &am, &av, &x_mean, &x_istd, &y_mean, &y_std, &X, &T,
                              &Z1, &A1, &Z2, &A2, &Z3, &A3, &dY, &dA, &dZ, &Xb, &Tb, &wpack, &red};
     for (auto* b : bufs) b->release();
-    idx.release();
+    orders.release();
     loss.release();
     if (stream) cudaStreamDestroy(stream);
   }
@@ -2954,24 +3001,33 @@ int adg_seed_train(adg_seed* s, int epochs, int batch, double lr, double* last_l
     int rc = seed_normalise(s);
     if (rc) return rc;
   }
-  if (seed_work(s, batch) != cudaSuccess || s->idx.ensure(s->nsamp) != cudaSuccess) return ADG_ERR_CUDA;
+  s->orders.train = s->stream;
+  if (seed_work(s, batch) != cudaSuccess || s->orders.ensure(s->nsamp) != cudaSuccess) return ADG_ERR_CUDA;
+  auto failed = [&] {  // nothing of this call is left running
+    cudaStreamSynchronize(s->orders.side);
+    cudaStreamSynchronize(s->stream);
+    return ADG_ERR_CUDA;
+  };
   std::vector<int> perm(s->nsamp);
   for (long long i = 0; i < s->nsamp; ++i) perm[i] = (int)i;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   for (int ep = 0; ep < epochs; ++ep) {
     std::shuffle(perm.begin(), perm.end(), s->rng);
-    cudaMemcpyAsync(s->idx.p, perm.data(), perm.size() * 4, cudaMemcpyHostToDevice, s->stream);
+    if (!send_order(s->orders, perm.data(), perm.size(), ep)) return failed();
+    const int* order = s->orders.order(ep & 1);
     cudaMemsetAsync(s->loss.p, 0, sizeof(double), s->stream);
     for (long long b0 = 0; b0 < s->nsamp; b0 += batch) {
       const int B = (int)std::min<long long>(batch, s->nsamp - b0);
-      if (seed_pass(s, s->X.p, s->T.p, s->idx.p + b0, B, s->stream) != cudaSuccess) return ADG_ERR_CUDA;
+      if (seed_pass(s, s->X.p, s->T.p, order + b0, B, s->stream) != cudaSuccess) return failed();
       s->adam_t++;
       const float bc1 = 1.f - (float)std::pow(b1, (double)s->adam_t), bc2 = 1.f - (float)std::pow(b2, (double)s->adam_t);
       mlp::k_adam<<<(unsigned)((s->nparam + 31) / 32), dim3(32, mlp::kSliceRows), 0, s->stream>>>(
           (int)s->nparam, s->params.p, slice_tab(s, B), s->red.p, s->am.p, s->av.p, (float)lr, b1, b2, eps, bc1, bc2);
     }
+    if (!s->orders.done(ep & 1)) return failed();
   }
-  // (one wait at the end: the next epoch's order is drawn while this one runs)
+  // (one wait at the end: the next epoch's order is drawn while this one runs,
+  // which is why an order is sent through buffers of its own)
   double l = 0.0;
   if (epochs > 0)
     cudaMemcpyAsync(&l, s->loss.p, sizeof(double), cudaMemcpyDeviceToHost, s->stream);
@@ -3003,7 +3059,10 @@ int adg_seed_gradients(adg_seed* s, const float* X, const float* T, int n, float
   cudaMemcpyAsync(s->Xb.p, X, (size_t)n * s->n_in * 4, cudaMemcpyHostToDevice, s->stream);
   cudaMemcpyAsync(s->Tb.p, T, (size_t)n * s->n_out * 4, cudaMemcpyHostToDevice, s->stream);
   cudaMemsetAsync(s->loss.p, 0, sizeof(double), s->stream);
-  if (seed_pass(s, s->Xb.p, s->Tb.p, nullptr, n, s->stream) != cudaSuccess) return ADG_ERR_CUDA;
+  if (seed_pass(s, s->Xb.p, s->Tb.p, nullptr, n, s->stream) != cudaSuccess) {
+    cudaStreamSynchronize(s->stream);  // the caller's X and T are no longer read
+    return ADG_ERR_CUDA;
+  }
   mlp::k_sum_slices<<<(unsigned)((s->nparam + 31) / 32), dim3(32, mlp::kSliceRows), 0, s->stream>>>(
       (int)s->nparam, slice_tab(s, n), s->red.p, s->grads.p);
   double l = 0.0;
