@@ -2746,13 +2746,14 @@ int seed_infer(adg_ctx* ctx, double* dst, int path, float* dst_f = nullptr) {
 }
 
 // Elements per block of the FP64 column kernels (mode 1, and mode 3's fallback
-// lists) where neither the caller nor the autotuner chose: not the plain
-// path's (a seeded step of 100^2 D2P3 with many elements falling back, 8 / 16:
-// 775 / 547 us).
+// lists): the caller's choice, else their own default, not what is chosen or
+// tuned for the plain path's kernel (a seeded step of 100^2 D2P3 with many
+// elements falling back, 8 / 16: 775 / 547 us).
 int column_elems(const adg_ctx* ctx) {
   const std::vector<int> ch = ctx->ks->elems_per_block_choices();
-  const int E = ctx->E_default ? (ctx->cfg.D == 2 ? 16 : 8) : ctx->E;
-  return std::find(ch.begin(), ch.end(), E) != ch.end() ? E : ctx->E;
+  auto built = [&](int E) { return std::find(ch.begin(), ch.end(), E) != ch.end(); };
+  const int own = ctx->cfg.elems_per_block, E = own > 0 && built(own) ? own : ctx->cfg.D == 2 ? 16 : 8;
+  return built(E) ? E : ctx->E;
 }
 // and of the seeded predictor
 int seeded_elems(const adg_ctx* ctx) {

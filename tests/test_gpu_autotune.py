@@ -55,3 +55,26 @@ def test_autotune_seeded_is_bitwise_neutral(tmp_path, monkeypatch):
     ua, ub = run(a, 6), run(b, 6)
     for x, y in zip(ua, ub):
         assert np.array_equal(x, y)
+
+
+def _cached(tmp_path, monkeypatch, lines):
+    """A context made with these lines of the cache file."""
+    f = tmp_path / "tune.txt"
+    f.write_text("".join(f"{k} {e}\n" for k, e in lines))
+    monkeypatch.setenv("ADG_TUNE_CACHE", str(f))
+    return make_gpu_amr("kh_p3_amr")
+
+
+def _key(tmp_path, monkeypatch):
+    """The key of the plain choice, as the library writes it."""
+    monkeypatch.setenv("ADG_TUNE_CACHE", str(tmp_path / "key.txt"))
+    make_gpu_amr("kh_p3_amr").autotune(1)
+    return (tmp_path / "key.txt").read_text().split()[0]
+
+
+@pytest.mark.parametrize("E", [8, 32])
+def test_fp64_columns_do_not_take_the_plain_choice(tmp_path, monkeypatch, E):
+    s = _cached(tmp_path, monkeypatch, [(_key(tmp_path, monkeypatch), E)])
+    G.PredictorSeed(2, 3, hidden=128, rng_seed=3).attach(s, mode=1, sweeps=2, tol=1e-3)
+    assert s.block_choices()["plain"] == E
+    assert s.block_choices()["seeded"] == 16
