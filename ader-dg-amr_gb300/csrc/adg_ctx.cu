@@ -169,8 +169,9 @@ struct adg_seed {
 struct adg_ctx {
   adg_config cfg{};
   const KernelSet* ks = nullptr;
-  int E = 0;  // elements per predictor block
-  bool E_default = true;  // neither the caller nor the autotuner chose E: it follows the layout's size
+  int E = 0;  // elements per predictor block of the plain path
+  bool E_follows = true;  // no choice of the caller's: E follows the layout's size
+  int E_tuned[2] = {};    // the autotuner's choice for layouts up to kFewElements and beyond (0: none)
   int sweeps = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -351,13 +352,20 @@ struct RemapTable {
   }
 };
 
+// E where the caller left it open.
+void choose_elems(adg_ctx* ctx) {
+  const long long n = (long long)ctx->hier.n_elem();
+  const int tuned = ctx->E_tuned[n > kFewElements];
+  ctx->E = tuned ? tuned : default_elems_per_block(*ctx->ks, n);
+}
+
 int upload_tables(adg_ctx* ctx, const RemapTable* rm = nullptr) {
   const Hierarchy& H = ctx->hier;
   const KernelSet* ks = ctx->ks;
   const int D = ctx->cfg.D, Q = ks->Q;
   const size_t ne = H.n_elem();
   const size_t nf = H.face_left.size();
-  if (ctx->E_default) ctx->E = default_elems_per_block(*ks, (long long)ne);
+  if (ctx->E_follows) choose_elems(ctx);
   ADG_CUDA(ctx->Rvol.ensure(ne * Q * ks->Np_s), "alloc Rvol");
   ADG_CUDA(ctx->Tr.ensure(ne * 2 * D * (size_t)ks->TR_TILE), "alloc traces");
   ADG_CUDA(ctx->Fnum.ensure(nf * Q * (size_t)ks->NM), "alloc Fnum");
@@ -1272,8 +1280,8 @@ int adg_ctx_create(const adg_config* cfg, adg_ctx** out) {
   ctx->sweeps = cfg->picard_sweeps > 0 ? cfg->picard_sweeps : cfg->P;
   if (ctx->sweeps < 1) ctx->sweeps = 1;
   std::vector<int> ch = ks->elems_per_block_choices();
-  ctx->E_default = !(cfg->elems_per_block > 0 && std::find(ch.begin(), ch.end(), cfg->elems_per_block) != ch.end());
-  ctx->E = ctx->E_default ? default_elems_per_block(*ks, 0) : cfg->elems_per_block;
+  ctx->E_follows = !(cfg->elems_per_block > 0 && std::find(ch.begin(), ch.end(), cfg->elems_per_block) != ch.end());
+  ctx->E = ctx->E_follows ? default_elems_per_block(*ks, 0) : cfg->elems_per_block;
   cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete ctx;
@@ -2249,10 +2257,15 @@ int adg_advance_timed_flushed(adg_ctx* ctx, int nsteps, int use_graph, int64_t f
 }
 
 // ---- autotuner: elements per block of the predictor stages ---------------
-// Per GPU model, (D, P), level-0 grid, finest level and stage, the fastest
+// Per GPU model, (D, P), level-0 grid, finest level, kernels and stage (the
+// plain one's also by the side of kFewElements the layout is on), the fastest
 // elements-per-block choice measured by adg_autotune, kept in a text file
 // (ADG_TUNE_CACHE, else $HOME/.cache/adg_gb300/tune.txt), one "key E" line each.
 namespace {
+
+// Part of every key: another value wherever the predictors change, so that a
+// choice is not taken for kernels it was not measured with.
+constexpr const char* kTunedKernels = "fixed-point-1";
 
 std::string tune_cache_path() {
   const char* p = std::getenv("ADG_TUNE_CACHE");
@@ -2261,7 +2274,7 @@ std::string tune_cache_path() {
   return std::string(h && *h ? h : "/tmp") + "/.cache/adg_gb300/tune.txt";
 }
 
-std::string tune_key(const adg_ctx* ctx, const char* stage) {
+std::string tune_key(const adg_ctx* ctx, const char* stage, int many = -1) {
   int dev = 0;
   cudaDeviceProp prop{};
   std::string gpu = "gpu";
@@ -2274,7 +2287,9 @@ std::string tune_key(const adg_ctx* ctx, const char* stage) {
   const adg_config& c = ctx->cfg;
   std::ostringstream k;
   k << gpu << "/D" << c.D << "P" << c.P << "/n" << c.n_cell[0] << "x" << (c.D > 1 ? c.n_cell[1] : 1) << "x"
-    << (c.D > 2 ? c.n_cell[2] : 1) << "/L" << c.max_level << "/" << stage;
+    << (c.D > 2 ? c.n_cell[2] : 1) << "/L" << c.max_level << "/" << kTunedKernels;
+  if (many >= 0) k << (many ? "/many" : "/few");
+  k << "/" << stage;
   return k.str();
 }
 
@@ -2319,10 +2334,9 @@ bool choice_built(const KernelSet* ks, int E) {
 static void apply_tuned_choices(adg_ctx* ctx) {
   if (ctx->cfg.elems_per_block > 0) return;
   int E = 0;
-  if (tune_lookup(tune_key(ctx, "plain"), &E) && choice_built(ctx->ks, E)) {
-    ctx->E = E;
-    ctx->E_default = false;
-  }
+  for (int many = 0; many < 2; ++many)
+    if (tune_lookup(tune_key(ctx, "plain", many), &E) && choice_built(ctx->ks, E)) ctx->E_tuned[many] = E;
+  if (ctx->E_follows && ctx->hier.n_elem()) choose_elems(ctx);
   if (ctx->seed_mode && tune_lookup(tune_key(ctx, ctx->seed_mode == 2 ? "seeded_fp32" : "seeded_fp64"), &E) &&
       choice_built(ctx->ks, E))
     ctx->Es = E;
@@ -2377,13 +2391,14 @@ int adg_autotune(adg_ctx* ctx, int nsteps, int* E_out, double* ms, int cap) {
   size_t best = 0;
   for (size_t i = 1; i < ch.size(); ++i)
     if (t[i] < t[best]) best = i;
+  const int many = (long long)ctx->hier.n_elem() > kFewElements;
   if (seeded) {
     ctx->Es = ch[best];
+    tune_store(tune_key(ctx, ctx->seed_mode == 2 ? "seeded_fp32" : "seeded_fp64"), ch[best]);
   } else {
-    ctx->E = ch[best];
-    ctx->E_default = false;
+    ctx->E = ctx->E_tuned[many] = ch[best];
+    tune_store(tune_key(ctx, "plain", many), ch[best]);
   }
-  tune_store(tune_key(ctx, seeded ? (ctx->seed_mode == 2 ? "seeded_fp32" : "seeded_fp64") : "plain"), ch[best]);
   ctx->graph_stale = true;  // the captured step used the old choice
   if (E_out) *E_out = ch[best];
   for (int i = 0; i < cap && ms; ++i) ms[i] = i < (int)ch.size() ? t[i] : 0.0;

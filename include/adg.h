@@ -359,8 +359,10 @@ int adg_time_kernels(adg_ctx* ctx, int nsteps, double* ms, int nkinds);
  * current layout, from a snapshot of the state that is restored afterwards
  * (the context's state, time, step count and counters are unchanged), keeps
  * the fastest in the context and records it per GPU model, (D, P), level-0
- * grid, finest level and stage (plain FP64, or the attached seed's mode) in
- * a text file: ADG_TUNE_CACHE, else $HOME/.cache/adg_gb300/tune.txt.
+ * grid, finest level and stage (plain, with the layout's element count up to or
+ * above 12288, or the attached seed's mode) in a text file: ADG_TUNE_CACHE,
+ * else $HOME/.cache/adg_gb300/tune.txt.  Entries of builds with other
+ * predictor kernels are not taken.
  * Contexts created with elems_per_block = 0 take the recorded choice at
  * adg_init and adg_seed_attach.  With a seed attached the seeded predictor is
  * tuned, else the plain one.  *E_out (may be NULL) receives the choice,
@@ -368,7 +370,9 @@ int adg_time_kernels(adg_ctx* ctx, int nsteps, double* ms, int nkinds);
  * the order of the configuration's choices.  No reference counterpart. */
 int adg_autotune(adg_ctx* ctx, int nsteps, int* E_out, double* ms, int cap);
 /* The elements-per-block choices the configuration is built with (up to cap)
- * and the ones in use by the plain and the seeded predictor. */
+ * and the ones in use by the plain and the seeded predictor.  (At D = 3, P <= 2
+ * the plain predictor's launch for the choice 8 has 6 elements a block, whose
+ * 30 columns fill a warp.) */
 int adg_block_choices(const adg_ctx* ctx, int* choices, int cap, int* n, int* E_plain, int* E_seeded);
 
 /* Page-locked host buffers for host<->device state copies. */

@@ -72,6 +72,19 @@ def _key(tmp_path, monkeypatch):
     return (tmp_path / "key.txt").read_text().split()[0]
 
 
+def test_entries_of_other_kernels_or_sizes_are_not_taken(tmp_path, monkeypatch):
+    """Some 700 elements, where the untuned choice is 8."""
+    key = _key(tmp_path, monkeypatch)
+    assert _cached(tmp_path, monkeypatch, [(key, 32)]).block_choices()["plain"] == 32
+    # the key of builds whose plain path was the FP64 column kernel
+    old = "/".join(key.split("/")[:5]) + "/plain"
+    assert old.endswith("/D2P3/n16x16x1/L2/plain")
+    assert _cached(tmp_path, monkeypatch, [(old, 32)]).block_choices()["plain"] == 8
+    many = key.replace("/few/", "/many/")
+    assert many != key
+    assert _cached(tmp_path, monkeypatch, [(many, 32)]).block_choices()["plain"] == 8
+
+
 @pytest.mark.parametrize("E", [8, 32])
 def test_fp64_columns_do_not_take_the_plain_choice(tmp_path, monkeypatch, E):
     s = _cached(tmp_path, monkeypatch, [(_key(tmp_path, monkeypatch), E)])
