@@ -5,6 +5,8 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "adg_fx.cuh"
+
 namespace adg {
 
 // Conversions between double and float, rounded to nearest even, in integer
@@ -64,39 +66,56 @@ constexpr uint32_t kStatusNaN = 1u;
 constexpr uint32_t kStatusNonPositiveDensity = 2u;
 constexpr uint32_t kStatusPressureFloor = 4u;
 
-// Reciprocal and square root with fewer FP64 operations: the FP32 estimate of
-// the significand (its bits moved by integer code; a conversion instruction
-// would occupy the FP64 pipe), then one third-order Householder step.  With
-// e = 1 - x r the estimate's relative error (about 2^-22),
+// Reciprocal and square root in integers, rounded as the operators round: the
+// FP32 estimate, whose relative error e is about 2^-22, one third-order
+// Householder step,
 //   1/x = r (1 + e + e^2 + ..), sqrt(x) = x r (1 + e/2 + 3 e^2/8 + ..),
-// whose next terms are below 2^-65: the results are within one unit in the
-// last place.  3 and 5 FP64 operations; outside 2^-900 .. 2^900 (zero,
-// infinities, NaN, negative square roots) the operators.
-__device__ __forceinline__ float significand_f32(int hi, int lo, int exp_bits) {
-  return __int_as_float(exp_bits | ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29));
+// to some units of 2^-60, then the exact remainder of the 54-bit quotient or
+// root decides its last bit.  (Neither is ever half way between two doubles.)
+// GB300 issues 1.6 FP64 operations a clock and SM.  The same steps in FP64 with
+// the residual correction that rounds them like this are 5 and 6 operations.
+// A pass of 32^2 D2P1 (20 steps) / 256^2 D2P3 / 64^3 D3P2, us: in FP64 633 /
+// 1265 / 9626, here 627 / 1229 / 9222; in FP64 without the correction (3 and 5
+// operations, one root in 20 rounded the other way) 616 / 1243 / 9484.
+// Outside 2^-900 .. 2^900 (zero, infinities, NaN, negative roots) the operators.
+__device__ __forceinline__ long long significand(int hi, int lo) {  // [2^52, 2^53)
+  return ((long long)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)lo;
 }
-__device__ __forceinline__ double widen_f32(float r, int exp_add, int sign) {
-  const int b = __float_as_int(r);
-  return __hiloint2double(((b >> 3) + (exp_add << 20)) | sign, b << 29);
+// m 2^(e - 52), m in [2^52, 2^53], as a double
+__device__ __forceinline__ double from_significand(long long m, int e, int sign) {
+  const long long b = m + ((long long)(e + 1022) << 52);
+  return __hiloint2double((int)(b >> 32) | sign, (int)b);
 }
 __device__ __forceinline__ double fast_rcp(double x) {
   const int hi = __double2hiint(x), ef = (hi >> 20) & 0x7ff;
   if ((unsigned)(ef - 123) > 1800u) return 1.0 / x;
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(significand_f32(hi, __double2loint(x), 0x3f800000)));
-  const double r0 = widen_f32(r, 1023 - 127 + 1023 - ef, hi & (int)0x80000000);
-  const double e = fma(-x, r0, 1.0);
-  return fma(r0, fma(e, e, e), r0);
+  const long long m = significand(hi, __double2loint(x));
+  // 2^106 / m within one of its whole part, then that: the remainder's low word holds it
+  long long q = fx_reciprocal(m << 7, 4) >> 6;
+  const long long rem = -(q * m);
+  q += (rem >= m) - (rem < 0);
+  return from_significand((q + 1) >> 1, 1022 - ef, hi & (int)0x80000000);
 }
 __device__ __forceinline__ double fast_sqrt(double x) {
   const int hi = __double2hiint(x), ef = hi >> 20;  // negative numbers: ef < 0
   if ((unsigned)(ef - 123) > 1800u) return sqrt(x);
-  const int k = ef - 1023, odd = k & 1;  // significand in [1, 4), even exponent
+  const int odd = (ef & 1) ^ 1;  // of the exponent ef - 1023: the significand, in [1, 4), takes it
+  const long long m = significand(hi, __double2loint(x)) << odd;
   float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(significand_f32(hi, __double2loint(x), 0x3f800000 + (odd << 23))));
-  const double r0 = widen_f32(r, 1023 - 127 - ((k - odd) >> 1), 0);
-  const double h = x * r0, e = fma(-h, r0, 1.0);
-  return fma(h, e * fma(0.375, e, 0.5), h);
+  asm("rsqrt.approx.ftz.f32 %0, %1;"
+      : "=f"(r)
+      : "f"(__int_as_float((0x3f800000 + (odd << 23)) | ((hi & 0xfffff) << 3) |
+                           (int)((unsigned)__double2loint(x) >> 29))));
+  const unsigned r0 = (unsigned)__float2int_rn(r * 16777216.0f);  // 2^24 r, exact
+  const long long g = (long long)(__umul64hi((unsigned long long)m << 10, (unsigned long long)r0 << 39) >> 2);  // 2^59 x r
+  const long long e = -(long long)((unsigned long long)g * r0);                            // 2^83 e
+  const int eh = (int)(e >> 32);
+  const long long c = (e >> 24) + 3 * (((long long)eh * eh) >> 45);                        // 2^60 (e/2 + 3 e^2/8)
+  // sqrt(2^54 m) within one of its whole part, then that
+  long long q = (g + __mul64hi(g << 1, c << 3)) >> 6;
+  const long long rem = (m << 54) - q * q;
+  q += (rem > 2 * q) - (rem < 0);
+  return from_significand((q + 1) >> 1, (ef - 1023 - odd) >> 1, 0);
 }
 __device__ __forceinline__ double reciprocal(double x) { return fast_rcp(x); }
 __device__ __forceinline__ float reciprocal(float x) { return 1.0f / x; }
