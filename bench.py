@@ -9,8 +9,9 @@ headline metric is quoted on.  A step is the whole evolve-loop body: regrid
 when due, ADER predictor-corrector of every element of every level in one
 launch per stage, reflux, average down, ghost fill, device time step.
 Metric: DOF-updates/s = sum over steps of valid elements of all levels times
-Q * Np_s.  The plain FP64 path and the learned-seed path run on the same
-workload; the headline value is the fastest seed variant whose L2 density
+Q * Np_s.  The plain path (named plain_fp64: FP64 state and fluxes, the
+predictor's operators in 60-bit fixed point) and the learned-seed path run on
+the same workload; the headline value is the fastest seed variant whose L2 density
 error against a converged-Picard FP64 run stays within 1.01x of the plain
 path's.
 
@@ -587,12 +588,21 @@ def e2e_device_patches(G, s, w, steps):
                     "device arrays with one ghost cell (AMReX FArrayBox layout)"}
 
 
-def roofline_line(G, w, workload, head_name, km_head, km_plain, el_per_step):
+def sm_count():
+    try:
+        import torch
+
+        return torch.cuda.get_device_properties(0).multi_processor_count, "this device's SMs"
+    except Exception:
+        return 152, "152 SMs (torch absent)"
+
+
+def roofline_line(G, w, workload, head_name, km_head, km_plain, el_per_step, clocks):
     """roofline of the headline path's dominant kernels: instruction issue (the
     ncu-counted warp instructions of one launch over the live CUDA-event
-    duration, against four a clock and SM at 2070 MHz), and beside it the FP64
-    pipe's (its instruction slots, 2 flops each, against the DFMA rate measured
-    in this run)."""
+    duration, against four a clock and SM at the SM clock sampled in this run),
+    and beside it the FP64 pipe's (its instruction slots, 2 flops each, against
+    the DFMA rate measured in this run)."""
     from math import comb
 
     D, P = w["D"], w["P"]
@@ -605,9 +615,12 @@ def roofline_line(G, w, workload, head_name, km_head, km_plain, el_per_step):
     key = "seeded_predictor" if seeded else "plain_predictor"
     t = km_head["seeded_predictor"] if seeded else km_plain["predictor"]
     prof = PROFILED_LAUNCH.get(workload, {}).get(key)
-    issue_peak = 4 * 152 * 2.07  # warp instructions per ns
+    sms, sms_source = sm_count()
+    mhz = (clocks or {}).get("sm_mhz") or 2070.0
+    issue_peak = 4 * sms * mhz * 1e-3  # G warp instructions/s
     line = {"bound": "issue", "unit": "G warp instructions/s", "peak": issue_peak,
-            "peak_source": "four schedulers on each of 152 SMs at the 2070 MHz of the sampled clocks",
+            "peak_source": f"four schedulers on each of {sms} SMs ({sms_source}) at {mhz:.0f} MHz "
+                           + ("(sampled in the timed region)" if (clocks or {}).get("sm_mhz") else "(no clock sample)"),
             "fp64_peak_tflops": peak,
             "fp64_peak_source": "FP64 DFMA-chain probe on this GPU in this run (adg_fp64_peak_probe; "
                                 "MEASURED_PEAKS.json has no FP64 figure)",
@@ -858,7 +871,7 @@ def run_ours(args, w):
     n_seed0 = G.seed_stats(head["sim"])[1] if seeded else 0
     km_head = head["sim"].time_kernels(3)
     el_per_step = plain["dof"] / args.steps / (Q * Nps)
-    roof = roofline_line(G, w, args.workload, head_name, km_head, km_plain, el_per_step)
+    roof = roofline_line(G, w, args.workload, head_name, km_head, km_plain, el_per_step, head["clocks"])
     if seeded and km_head.get("seed_inference", 0.0) > 0.0:
         # the seed network runs over every element of the layout, the
         # coarse-fine ghosts included: its count over the same three steps
@@ -868,9 +881,12 @@ def run_ours(args, w):
         "metric": METRIC, "value": value, "unit": "DOF-updates/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64" if head_name == "plain_fp64" else "f64+f32",
-        "dtype_detail": (None if head_name == "plain_fp64" else
-                         "FP64 state, corrector, numerical-flux moments and the time-independent part of the "
-                         "predictor; FP32 Picard sweeps and flux changes; TF32 tensor-core seed network"),
+        "dtype_detail": ("FP64 state, corrector, numerical flux, final-stage fluxes and face physics; predictor "
+                         "operators and the sweeps' fluxes in 60-bit fixed point with one exponent per column"
+                         if head_name == "plain_fp64" else
+                         "FP64 state, corrector and numerical-flux moments; the time-independent part of the "
+                         "predictor in 60-bit fixed point; FP32 Picard sweeps and flux changes; TF32 tensor-core "
+                         "seed network"),
         "data": "synthetic",
         "config": base_config(args, w, world),
         "run": {"path": head_name, "autotune": {"plain": tune, "seeded": tune_seeded}, "cuda_graph": True,
