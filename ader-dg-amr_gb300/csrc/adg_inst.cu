@@ -132,8 +132,8 @@ cudaError_t launch_predictor(const PredictorArgs& a, cudaStream_t s, int mode) {
 
 // Elements per block of the plain-only configurations: whole warps of columns
 // at D = 2 (a block of 16 at P = 6 needs 214 KB of shared memory), at D = 3
-// what leaves two blocks on an SM (P = 3, 20 x 14 x 18: 4 / 6 elements 692 /
-// 737 us).
+// what leaves two blocks on an SM (P = 3, 20 x 14 x 18: 4 / 6 elements 641 /
+// 656 us).
 constexpr int lite_elems() { return O::D == 2 ? 8 : 4; }
 
 struct Impl final : KernelSet {
@@ -169,7 +169,8 @@ struct Impl final : KernelSet {
   }
 #else
   // (the plain path takes 6 elements for the choice 8: 30 columns fill a warp
-  // and its table reads are uniform; P = 2, 64^3: 9.0 -> 8.5 ms)
+  // and its table reads are uniform; the kernel with 8 / 6: P = 2, 64^3 7.54 /
+  // 7.42 ms, 20^3 284 / 262 us; P = 1, 32^3 168 / 176 us)
   std::vector<int> elems_per_block_choices() const override { return {4, 8, 16}; }
   size_t predictor_smem(int E) const override {
     return E == 4 ? FxShape<O, 4>::BYTES : E == 8 ? FxShape<O, 6>::BYTES : FxShape<O, 16>::BYTES;

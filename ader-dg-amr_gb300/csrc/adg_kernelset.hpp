@@ -66,8 +66,8 @@ const KernelSet* kernels_D2P6();
 const KernelSet* kernels_D3P3();
 
 // Elements per block where nothing else chose them.  D = 2: blocks of 8 while
-// blocks of 16 leave the SMs with a few blocks each (D2P3 step, us, 8 / 16:
-// 24^2 86 / 101, 48^2 96 / 102; 128^2 329 / 332; 256^2 1220 / 1169).
+// blocks of 16 leave the SMs with a few blocks each (D2P3, a whole step, us, 8 /
+// 16: 24^2 82 / 92, 48^2 89 / 94; 128^2 344 / 334; 256^2 1236 / 1137).
 constexpr long long kFewElements = 12288;
 inline int default_elems_per_block(const KernelSet& ks, long long n_elem) {
   const std::vector<int> ch = ks.elems_per_block_choices();

@@ -27,7 +27,7 @@
 // column-per-thread FP64 predictor kept that pipe 84 % busy; with the
 // operators on the integer pipes it still set the time through the fluxes
 // (D2P3, 256^2: 2330 -> 1169 us), and with integer fluxes in the sweeps the
-// kernel issues 2.0 instructions per clock and SM (1169 -> 1000 us; a flux
+// kernel issues 2.0 instructions per clock and SM (1169 -> 1010 us; a flux
 // costs the integer pipes what its conversions cost before).  Now: dependent
 // integer chains and the barriers between phases.  The stages are short loops
 // over tables instead of unrolled code per (operator, time node):
@@ -53,10 +53,12 @@ struct FxShape {
   static constexpr int ROWS = (NP_ST + LINES - 1) / LINES;            // rows of H_w per thread
   static constexpr int TASKS = (D * O::FX_NPRE + LINES - 1) / LINES;  // (direction, mode prefix) per thread
   static constexpr int PTS = (E * NS + NT - 1) / NT;                  // points per thread
-  // warps per SM that the register limit allows: the phases wait at barriers
-  // and on the FP64 pipe, so more blocks beat a few spills (D2P3, 256^2:
-  // 16 / 24 / 32 warps 1330 / 1169 / 1216 us; D3P2, 64^3: 11.9 / 9.0 / 8.5
-  // ms), except where a line is long (D2P6 spills 300 bytes at 24)
+  // warps per SM that the register limit allows: the phases wait at barriers,
+  // so more blocks beat a few spills (the kernel at 16 / 24 / 32 warps: D2P3,
+  // 256^2, 1163 / 1010 / 1068 us, 104 bytes spilled at 24; D3P2, 64^3, 13.3 /
+  // 8.3 / 7.4 ms, 232 bytes at 32; D3P3, 20 x 14 x 18, 1007 / 691 / 652 us,
+  // 392 bytes), except where a line is long (D2P4, 100^2, 625 / 691 / 822 us;
+  // D2P6, 48^2, 851 / 1004 / 1022, 204 bytes at 16)
   static constexpr int WARPS = D == 3 ? 32 : N <= 4 ? 24 : 16;
   static constexpr int MIN_BLOCKS = WARPS * 32 / NT > 0 ? WARPS * 32 / NT : 1;
   // 64-bit slots: modes, U, g, fluxes, accumulators

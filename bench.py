@@ -365,13 +365,13 @@ PROFILED_LAUNCH = {
     "kh_p3_amr3": {
         "plain_predictor": dict(kernel="k_predictor_fx<D2P3, E=8> (3 Picard sweeps in fixed point, corrector volume "
                                        "term, face traces)",
-                                inst=165.907e6, fp64_pipe_slots=52.345e6, fp64_arith=49.347e6, dram_bytes=29.95e6,
-                                issue_active=0.485, fp64_active=0.305, elements=15616,
+                                inst=171.249e6, fp64_pipe_slots=41.351e6, fp64_arith=38.353e6, dram_bytes=31.01e6,
+                                issue_active=0.502, fp64_active=0.242, elements=15616,
                                 source="profiles/fp64_issue_k_predictor_kh_p3_amr3.md"),
         "seeded_predictor": dict(kernel="k_split_base<D2P3, E=8> (time-independent part in fixed point) and "
                                         "k_predictor<D2P3, E=8, MODE 2> (2 FP32 sweeps from the seed, FP32 changes)",
-                                 inst=37.752e6, fp64_pipe_slots=5.309e6, fp64_arith=3.670e6, dram_bytes=29.52e6,
-                                 issue_active=0.442, fp64_active=0.122, elements=15616,
+                                 inst=38.176e6, fp64_pipe_slots=5.309e6, fp64_arith=3.670e6, dram_bytes=29.57e6,
+                                 issue_active=0.443, fp64_active=0.121, elements=15616,
                                  source="profiles/fp64_issue_k_predictor_kh_p3_amr3.md"),
     },
 }

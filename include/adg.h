@@ -408,7 +408,11 @@ int adg_seed_gradients(adg_seed* s, const float* X, const float* T, int n, float
 int adg_seed_num_params(const adg_seed* s, int64_t* n_weights, int64_t* n_total);
 int adg_seed_get_params(adg_seed* s, float* out);
 int adg_seed_set_params(adg_seed* s, const float* in);
-/* mode 0 detaches; 1: sweeps in FP64; 2: sweeps in FP32. */
+/* mode 0 detaches; 1: sweeps in FP64; 2: sweeps in FP32.  Mode 1 and the
+ * fallback of mode 2 run FP64 column kernels: on the benchmark workload one
+ * mode-1 sweep takes longer than the plain path's three (1.26e9 against 1.81e9
+ * DOF-updates/s), so mode 1 saves no time, and mode 2 does where few elements
+ * fall back (adg_seed_stats). */
 int adg_seed_attach(adg_ctx* ctx, adg_seed* s, int mode, int sweeps, double tol);
 /* Which kernels compute the seed during steps: 1 (default) the fused
  * tensor-core kernel (features, the four layers as TF32 tcgen05 MMAs with
